@@ -53,6 +53,14 @@ static inline uint32_t tiles_for(uint32_t n) { return (n + 63) / 64; }
 
 // Iterations of a persistent closure whose phase timestamps are kept.
 constexpr uint32_t kPhaseLogIters = 4096;
+// Work items per CTA of a persistent iteration above which a late-selecting
+// closure goes on in the multi-kernel loop.  That loop costs ~25 us per
+// iteration instead of ~12, and gives dense iterations merged rules and the
+// tensor cores: random CNF at n = 3001 12.5 -> 4.1 ms, n = 1800 3.7 -> 1.8 ms.
+// Same-generation at n = 8192 never passes 2 per CTA.  Limits of 3, 6, 12, 30
+// on closures that are heavy only for a while (random CNF, grammar 5, n = 1800):
+// 1948, 1224, 1277, 1237 us; on dense ones (n = 900) 649, 656, 690, 817 us.
+constexpr uint32_t kLeaveItems = 12;
 // Iterations of a closure whose selection rows are kept.
 constexpr uint32_t kSelLogIters = 128;
 
@@ -1027,6 +1035,11 @@ struct ClosurePlan {
     uint32_t tc_groups = 0;       // groups of 4 tile-rows over all tensor-core-capable products
     uint32_t tc_max_T = 0;
     bool auto_select = false;     // variants chosen on the device every iteration
+    // A single AUTO query below the selector's size: it starts in the
+    // persistent kernel with LOP3 throughout, and goes on with selection in
+    // the multi-kernel loop if its iterations turn out heavy (the tables of
+    // both stages are kept).
+    bool late_select = false;
     uint8_t fixed_variant = 0;    // otherwise: every product's variant
     std::vector<uint8_t> tc_ok;   // per product: has a tensor-core launch sequence
     std::vector<QueryRange> qranges;  // per query: its plan rows, slot rows, slots and products
@@ -1093,8 +1106,10 @@ static int build_plan(cfpq_ctx *ctx, const std::vector<QueryIn> &qs, int variant
     for (const QueryIn &q : qs)
         if (q.nmats && q.nrules) max_T = std::max(max_T, q.mats[0]->d.T);
     // a single small query is latency-bound: selection costs more than it gains
-    pl->auto_select = variant == CFPQ_VARIANT_AUTO && ctx->sel.mode != CFPQ_SELECT_FIXED &&
-                      (allowed & ~(1u << CFPQ_VARIANT_LOP3)) != 0 && (qs.size() > 1 || max_T >= ctx->sel.min_tiles);
+    const bool selects = variant == CFPQ_VARIANT_AUTO && ctx->sel.mode != CFPQ_SELECT_FIXED &&
+                         (allowed & ~(1u << CFPQ_VARIANT_LOP3)) != 0;
+    pl->auto_select = selects && (qs.size() > 1 || max_T >= ctx->sel.min_tiles);
+    pl->late_select = selects && !pl->auto_select;
     pl->fixed_variant = (uint8_t)(variant == CFPQ_VARIANT_M4R || variant == CFPQ_VARIANT_TC ? variant
                                                                                            : CFPQ_VARIANT_LOP3);
     const bool tc_auto = (allowed & (1u << CFPQ_VARIANT_TC)) != 0;
@@ -1149,8 +1164,8 @@ static int build_plan(cfpq_ctx *ctx, const std::vector<QueryIn> &qs, int variant
                 // may run on tensor cores also plans ceil(T/4) groups of 4
                 // tile-rows from the same start in its own launch
                 pd.row_start = pl->prod_rows;
-                const bool tc = pl->auto_select ? tc_auto && T >= ctx->sel.tc_min_tiles
-                                                : pl->fixed_variant == CFPQ_VARIANT_TC;
+                const bool tc = pl->auto_select || pl->late_select ? tc_auto && T >= ctx->sel.tc_min_tiles
+                                                                   : pl->fixed_variant == CFPQ_VARIANT_TC;
                 if (tc) {
                     pl->tc_prods.push_back(TcProduct{(uint32_t)pl->prods.size(), T, pl->prod_rows, (T + 3) / 4});
                     pl->tc_max_T = std::max(pl->tc_max_T, T);
@@ -1168,7 +1183,7 @@ static int build_plan(cfpq_ctx *ctx, const std::vector<QueryIn> &qs, int variant
         pl->qranges.push_back(qrange);
     }
     pl->item_cap = std::max<size_t>(pl->item_cap, 1);
-    pl->uses_tc = !pl->tc_prods.empty();
+    pl->uses_tc = !pl->tc_prods.empty() && !pl->late_select;
     for (const TcProduct &tp : pl->tc_prods) {
         pl->tc_rows.push_back(TcRows{tp.index, tp.row_start, pl->tc_groups, 0});
         pl->tc_groups += tp.rows;
@@ -1222,7 +1237,7 @@ static BufCounters *closure_counters(cfpq_ctx *ctx, const ClosurePlan &) {
 static int enqueue_select_plan(cfpq_ctx *ctx, const ClosurePlan &pl, const QueryTrack &qt, cudaStream_t s) {
     const PlanSelect ps = {ctx->d_sel.as<SelectorParams>(), ctx->cnts.as<BufCounters>(), ctx->tc_ok.as<uint8_t>(),
                            ctx->choice.as<uint8_t>(), ctx->sel_log_iters ? ctx->sel_log.as<SelLogRow>() : nullptr,
-                           ctx->sel_log_iters};
+                           ctx->sel_log_iters, nullptr, 1};
     CUDA_TRY(launch_plan(ctx->prods.as<ProdDesc>(), (uint32_t)pl.prods.size(), 0, pl.prod_rows,
                          ctx->slots.as<MatSlot>(), ctx->d_st, ctx->items.as<uint64_t>(), pl.item_cap,
                          product_lop3_tiles_per_block(), ctx->prod_seen.as<uint32_t>(), 0, ctx->choice.as<uint8_t>(),
@@ -1235,7 +1250,7 @@ static int enqueue_select_plan(cfpq_ctx *ctx, const ClosurePlan &pl, const Query
 static int enqueue_products(cfpq_ctx *ctx, const ClosurePlan &pl, const QueryTrack &qt, cudaStream_t s) {
     BufCounters *cnts = closure_counters(ctx, pl);
     TRY(launch_products(ctx, pl.item_cap, pl.uses_lop3, pl.uses_m4r, qt.changed, cnts, s));
-    if (!pl.tc_prods.empty()) {
+    if (pl.uses_tc) {
         // every tensor-core product of the iteration together: one plan
         // launch, one tensor-core launch over all their items, one list reset
         const ProdDesc *pr = ctx->prods.as<ProdDesc>();
@@ -1410,7 +1425,7 @@ static int run_logged_iterations(cfpq_ctx *ctx, const ClosurePlan &pl, const Que
         ctx->tev.push_back(e);
     }
     std::vector<int> tc_index(np, -1);
-    for (size_t i = 0; i < pl.tc_prods.size(); ++i) tc_index[pl.tc_prods[i].index] = (int)i;
+    for (size_t i = 0; pl.uses_tc && i < pl.tc_prods.size(); ++i) tc_index[pl.tc_prods[i].index] = (int)i;
     std::vector<SelLogRow> rows(np);
     for (uint32_t it = 0;; ++it) {
         if (it > (1u << 20)) return set_error(CFPQ_ERR_CUDA, "closure did not converge");
@@ -1512,6 +1527,39 @@ static void fill_hash_out(const cfpq_ctx *ctx, const HashOut *ho) {
         ho->hashes[i] = ctx->h_hash[2 * i] % 1000000007ULL;
         ho->counts[i] = ctx->h_hash[2 * i + 1];
     }
+}
+
+// Second stage of a late-selecting closure (ClosurePlan::late_select) whose
+// iterations became heavy: the persistent kernel has left after iteration
+// st->iter - 1 with the deltas ready for the next one; the counters are
+// measured and the multi-kernel loop with selection runs
+// to the fixpoint (result lines wanted are hashed again).
+static int finish_selected(cfpq_ctx *ctx, ClosurePlan &pl, const QueryTrack &qt, uint32_t nslots, const HashOut *ho) {
+    struct Stage {  // the plan's selecting view, put back on every way out
+        cfpq_ctx *ctx;
+        ClosurePlan &pl;
+        bool lop3, m4r;
+        ~Stage() {
+            pl.auto_select = pl.uses_tc = ctx->cnts_on = false;
+            pl.uses_lop3 = lop3;
+            pl.uses_m4r = m4r;
+        }
+    } stage{ctx, pl, pl.uses_lop3, pl.uses_m4r};
+    pl.auto_select = ctx->cnts_on = true;
+    pl.uses_tc = !pl.tc_prods.empty();
+    pl.uses_lop3 = true;
+    pl.uses_m4r = (ctx->sel.allowed & (1u << CFPQ_VARIANT_M4R)) != 0;
+    TRY(selector_sync(ctx));
+    CUDA_TRY(cudaMemsetAsync(qt.changed, 0, 3 * sizeof(uint32_t), ctx->stream));
+    CUDA_TRY(launch_counters_init(ctx->slots.as<MatSlot>(), nslots, ctx->cnts.as<BufCounters>(), true, ctx->stream));
+    cudaGraphExec_t exec = nullptr;
+    TRY(get_loop_graph(ctx, pl, qt, &exec));
+    CUDA_TRY(cudaGraphLaunch(exec, ctx->stream));
+    CUDA_TRY(cudaEventRecord(ctx->ev1, ctx->stream));
+    CUDA_TRY(cudaMemcpyAsync(ctx->h_st, ctx->d_st, sizeof(IterState), cudaMemcpyDeviceToHost, ctx->stream));
+    if (ho && ho->n) TRY(enqueue_hash_many(ctx, ho->mats, ho->n));
+    CUDA_TRY(cudaStreamSynchronize(ctx->stream));
+    return CFPQ_OK;
 }
 
 static int run_engine(cfpq_ctx *ctx, const std::vector<QueryIn> &qs, const cfpq_closure_opts &o,
@@ -1643,11 +1691,10 @@ static int run_engine(cfpq_ctx *ctx, const std::vector<QueryIn> &qs, const cfpq_
     // touches neither the matrices nor the counters
     if (input) CUDA_TRY(launch_closure_input(*input, ctx->num_sms, ctx->stream, &b));
     if (ctx->cnts_on) CUDA_TRY(launch_counters_init(ctx->slots.as<MatSlot>(), nslots, ctx->cnts.as<BufCounters>(),
-                                                    ctx->stream));
+                                                    false, ctx->stream));
     if (ctx->sel_log_iters)
         CUDA_TRY(cudaMemsetAsync(ctx->sel_log.p, 0, (size_t)kSelLogIters * nprods * sizeof(SelLogRow), ctx->stream));
     if (!input) CUDA_TRY(launch_closure_begin(b, ctx->num_sms, ctx->stream));
-
     cudaGraphExec_t exec = nullptr;
     if (o.use_graph && !timed && !log_products && !persistent) TRY(get_loop_graph(ctx, pl, qt, &exec));
     if (timed) memset(&ctx->prof, 0, sizeof(ctx->prof));
@@ -1685,6 +1732,7 @@ static int run_engine(cfpq_ctx *ctx, const std::vector<QueryIn> &qs, const cfpq_
                                            nq == 1 && pl.prods[0].T <= kDirectMergeMaxTiles ? 1 : 0,
                                            nq > 1 ? 1 : 0, (uint32_t)std::max(o.wait_limit, 0),
                                            (o.test_flags & CFPQ_TEST_STALL_BARRIER) != 0,
+                                           pl.late_select && !o.log_products ? kLeaveItems : 0u,
                                            st_mapped ? ctx->h_st_dev : nullptr,
                                            flag_mapped ? ho->flag_src : nullptr,
                                            flag_mapped ? ctx->h_flag_dev + (ho->flag_dst - ctx->h_flag) : nullptr,
@@ -1733,16 +1781,19 @@ static int run_engine(cfpq_ctx *ctx, const std::vector<QueryIn> &qs, const cfpq_
     if (ho && ho->flag_src && !flag_mapped)
         CUDA_TRY(cudaMemcpyAsync(ho->flag_dst, ho->flag_src, 4, cudaMemcpyDeviceToHost, ctx->stream));
     CUDA_TRY(cudaStreamSynchronize(ctx->stream));
+    const IterState &hs = *ctx->h_st;
+    ctx->phase_log_iters = persistent ? std::min<uint32_t>(hs.iter, kPhaseLogIters) : 0;
+    const uint32_t persistent_iters = persistent ? hs.iter : 0;
+    const bool left = persistent && hs.left && !hs.error;
+    if (left) TRY(finish_selected(ctx, pl, qt, nslots, ho));
     float ms = 0;
     CUDA_TRY(cudaEventElapsedTime(&ms, ctx->ev0, ctx->ev1));
-    const IterState &hs = *ctx->h_st;
     const bool converged = hs.last_changed == 0;
-    ctx->phase_log_iters = persistent ? std::min<uint32_t>(hs.iter, kPhaseLogIters) : 0;
     if (hs.error) {
         drop_plan_cache(ctx, true);
         return set_error(CFPQ_ERR_TIMEOUT, "a bounded device wait gave up during the closure");
     }
-    if (persistent) {
+    if (persistent && !left) {
         ctx->items_clean_ptr = ctx->items.p;
         ctx->items_clean_words = list_words;
     }
@@ -1760,8 +1811,9 @@ static int run_engine(cfpq_ctx *ctx, const std::vector<QueryIn> &qs, const cfpq_
         // the counters, the prologue when it ran alone, the closure, the hash
         const uint64_t input_launches = input ? 1 + (input->nedges ? 1 : 0) + (input->ndiag ? 1 : 0) : 0;
         stats->kernel_launches = input_launches + (ctx->cnts_on ? 1 : 0) + (input ? 0 : 1) +
-                                 (persistent ? 1 : (uint64_t)hs.iter * 3) +
-                                 (ho && ho->n ? (ho->n + kHashBatch - 1) / kHashBatch : 0);
+                                 (persistent ? 1 + (uint64_t)(hs.iter - persistent_iters) * 3 : (uint64_t)hs.iter * 3) +
+                                 (ho && ho->n ? (ho->n + kHashBatch - 1) / kHashBatch * (left ? 2 : 1) : 0) +
+                                 (left ? 1 : 0);
         stats->variant_items[CFPQ_VARIANT_LOP3] = hs.items_by_variant[2];
         stats->variant_items[CFPQ_VARIANT_M4R] = hs.items_by_variant[3];
         stats->variant_items[CFPQ_VARIANT_TC] = hs.items_by_variant[4];

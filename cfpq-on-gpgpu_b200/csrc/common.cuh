@@ -83,7 +83,7 @@ struct IterState {
     alignas(128) uint32_t pitem_next[2][2];
     // grid barrier of the iterations of parity p: low 32 bits count the CTAs'
     // arrivals (cumulative over the closure), high 32 bits are the
-    // iteration's flags (kBarChanged, kBarAbort), read with the count
+    // iteration's flags (kBarChanged ..), read with the count
     alignas(128) unsigned long long pbar[2];
     unsigned long long tile_triples;
     unsigned long long items_total;
@@ -95,6 +95,7 @@ struct IterState {
     unsigned long long out_words;     // non-zero accumulator words merged into heads
     unsigned long long new_words;     // words that received new bits
     uint32_t exit_count;              // persistent kernel: CTAs past their exit statistics
+    uint32_t left;                    // persistent kernel: left before the fixpoint (kBarLeave), still active
 };
 
 // A matrix and the prefix sum of tile-rows over a list of matrices (kernels
@@ -161,10 +162,17 @@ struct PlanSelect {
     // (1-based) in which it changed; a query that did not change in the
     // previous iteration has empty deltas and is not planned
     const uint32_t *q_last;
+    // no product runs while this plan does (multi-kernel iterations), so the
+    // counters of the current matrices are the same for every planning warp
+    int static_counts;
 };
 
-constexpr uint32_t kBarChanged = 1u;  // some product set a new bit
-constexpr uint32_t kBarAbort = 2u;    // a CTA gave up a bounded wait
+// Flags of the barrier word, one byte each: kBarChanged is set by plain byte
+// stores (every merging warp does it; atomics on one word would serialise),
+// the rare others by an atomic OR, and neither disturbs the other.
+constexpr uint32_t kBarChanged = 1u;       // some product set a new bit
+constexpr uint32_t kBarAbort = 1u << 8;    // a CTA gave up a bounded wait
+constexpr uint32_t kBarLeave = 1u << 16;   // many items per CTA: the closure goes on in the multi-kernel loop
 
 // Rows, slots and products of one query of a closure (all contiguous): plan
 // rows [prow0, prow0 + nprow), slot tile-rows [srow0, srow0 + nsrow), slots
@@ -211,7 +219,15 @@ __device__ __forceinline__ unsigned long long globaltimer_ns() {
 // k-tile that appears during the iteration may be processed or not: its bits
 // are also in the next delta).  Items of the same output block are
 // independent: their partial products are OR-ed into the head atomically.
-// Fields: p 16 bits, ti 11, tjb 9, klo 12, khi 12 (T <= 2048).
+// Fields: p 16 bits, ti 11, tjb 9, klo 12, khi 12 (T <= 2048), flags 4.
+//
+// Flags: kItemM4R (persistent kernel: Four Russians inner loop); kItemMerged:
+// the item belongs to a merged rule -- one product of the current matrices
+// that stands for both of the rule's terms (sel::merge_terms) and visits a
+// k-tile only if its P tile or its Q block holds bits of the delta.
+constexpr uint32_t kItemM4R = 1u;
+constexpr uint32_t kItemMerged = 2u;
+constexpr uint32_t kChoiceMerged = 0x80;  // choice[] of a merged rule's first term: variant | kChoiceMerged
 constexpr uint32_t kMaxItemProducts = 1u << 16;
 __host__ __device__ inline uint64_t make_item(uint32_t p, uint32_t ti, uint32_t tjb, uint32_t klo, uint32_t khi) {
     return ((uint64_t)p << 48) | ((uint64_t)ti << 37) | ((uint64_t)tjb << 28) | ((uint64_t)klo << 16) |

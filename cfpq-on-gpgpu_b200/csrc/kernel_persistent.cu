@@ -40,6 +40,9 @@
 // semi-naive terms of its planner, and bits it finds beyond those are true
 // and recorded in the delta like any other.
 //
+// Closures without Four Russians items never merge rules (kItemMerged is the
+// selection's, and selection comes with Four Russians).
+//
 // The same plan and item code as the multi-kernel iteration runs here; only
 // the sequencing differs.  Every wait is bounded: a CTA that gives up sets
 // the error word and leaves the loop, and every other wait then gives up too.
@@ -128,6 +131,8 @@ struct PersistArgs {
     uint32_t spin_limit;            // polls of the item wait and of the grid barrier before they give up
     uint32_t stall_barrier;         // test hook: the first grid barrier waits for one arrival more than
                                     // there are CTAs, so that its bounded wait runs out
+    uint32_t leave_idx;             // after an iteration that has an item of this list index the kernel leaves, the
+                                    // closure's state ready for the multi-kernel loop's next iteration
     IterState *host_st;             // non-null: the last CTA to exit writes the final state here
     const uint32_t *flag_src;       // and (non-null) this word to *flag_dst (both mapped host memory)
     uint32_t *flag_dst;
@@ -263,9 +268,10 @@ __global__ void __launch_bounds__(kThreads, 2) k_closure_persistent(PersistArgs 
         prods = reinterpret_cast<const ProdDesc *>(S.tables + slot_bytes);
     }
     __syncthreads();
-    const PlanSelect psel = {a.sel && a.cnts ? a.sel : nullptr, a.cnts, nullptr, a.choice, a.sel_log, a.sel_log_iters};
+    const PlanSelect psel = {a.sel && a.cnts ? a.sel : nullptr, a.cnts, nullptr, a.choice, a.sel_log, a.sel_log_iters,
+                             nullptr, 0};
     uint32_t phase = 0, bar_uses[2] = {0, 0};
-    bool timed_out = false;
+    bool timed_out = false, left = false;
     ItemCounters ctr;
     const uint32_t iter0 = st->iter, max_iter = st->max_iter;
     uint32_t t = iter0;
@@ -310,10 +316,10 @@ __global__ void __launch_bounds__(kThreads, 2) k_closure_persistent(PersistArgs 
                 if (u < np) {
                     const uint32_t i = active_find(X.act_plan, u);
                     const QueryRange qr = a.qr[X.act_plan.q[i]];
-                    plan::plan_row(qr.prow0 + (u - X.act_plan.pref[i]), prods, a.nprods, slots, t, st,
-                                   item_count, items, a.list_cap, a.tpb, a.prod_seen, 0, psel,
-                                   X.plan[warp].cnt, X.plan[warp].bnd, qr.prod0, qr.prod0 + qr.nprod,
-                                   &st->pitem_m4r[par]);
+                    plan::plan_row<kHasM4R>(qr.prow0 + (u - X.act_plan.pref[i]), prods, a.nprods, slots, t, st,
+                                            item_count, items, a.list_cap, a.tpb, a.prod_seen, 0, psel,
+                                            X.plan[warp].cnt, X.plan[warp].bnd, qr.prod0, qr.prod0 + qr.nprod,
+                                            &st->pitem_m4r[par]);
                 } else {
                     const uint32_t i = active_find(X.act_clear, u - np);
                     const QueryRange qr = a.qr[X.act_clear.q[i]];
@@ -327,9 +333,9 @@ __global__ void __launch_bounds__(kThreads, 2) k_closure_persistent(PersistArgs 
             const uint32_t units = a.prod_rows + clear_rows;
             for (uint32_t u = gwarp; u < units; u += nwarps) {
                 if (u < a.prod_rows) {
-                    plan::plan_row(u, prods, a.nprods, slots, t, st, item_count, items, a.list_cap, a.tpb,
-                                   a.prod_seen, 0, psel, X.plan[warp].cnt, X.plan[warp].bnd, 0u, 0xFFFFFFFFu,
-                                   &st->pitem_m4r[par]);
+                    plan::plan_row<kHasM4R>(u, prods, a.nprods, slots, t, st, item_count, items, a.list_cap, a.tpb,
+                                            a.prod_seen, 0, psel, X.plan[warp].cnt, X.plan[warp].bnd, 0u, 0xFFFFFFFFu,
+                                            &st->pitem_m4r[par]);
                 } else {
                     clear_delta_row(slots, a.nslots, u - a.prod_rows, par ^ 1);
                 }
@@ -386,6 +392,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_closure_persistent(PersistArgs 
                 }
                 if (v) {
                     *slot = 0;
+                    if (idx == a.leave_idx) atomicOr(changed, kBarLeave);
                     // batches: take the next index now, its round trip
                     // overlaps this item (a single closure keeps items for
                     // the CTAs that are free first)
@@ -404,19 +411,19 @@ __global__ void __launch_bounds__(kThreads, 2) k_closure_persistent(PersistArgs 
             }
             const unsigned long long t0 = a.trace ? globaltimer_ns() : 0ull;
             unsigned long long sub[4] = {t0, t0, t0, t0};
-            const uint64_t item = v & ~1ull;
+            const uint64_t item = v & ~(unsigned long long)kItemM4R;
             bool m4r_item = false;
-            if constexpr (kHasM4R) m4r_item = (v & 1ull) != 0;
+            if constexpr (kHasM4R) m4r_item = (v & kItemM4R) != 0;
             if constexpr (kHasM4R) {
                 if (m4r_item)
-                    tiled::process_item<true, kPW>(S.prod, item, prods, slots, t, changed, qchanged,
-                                                   phase, timed_out, ctr, a.cnts, &gate, gridDim.x,
-                                                a.direct_merge != 0, a.trace ? sub : nullptr);
+                    tiled::process_item<true, kPW, kHasM4R>(S.prod, item, prods, slots, t, changed, qchanged, phase,
+                                                            timed_out, ctr, a.cnts, &gate, gridDim.x,
+                                                            a.direct_merge != 0, a.trace ? sub : nullptr);
             }
             if (!m4r_item)
-                tiled::process_item<false, kPW>(S.prod, item, prods, slots, t, changed, qchanged, phase,
-                                                timed_out, ctr, a.cnts, &gate, gridDim.x,
-                                                a.direct_merge != 0, a.trace ? sub : nullptr);
+                tiled::process_item<false, kPW, kHasM4R>(S.prod, item, prods, slots, t, changed, qchanged, phase,
+                                                         timed_out, ctr, a.cnts, &gate, gridDim.x,
+                                                         a.direct_merge != 0, a.trace ? sub : nullptr);
             if (a.trace && tid == 0) trace_item(a, item, t, (uint32_t)(v & 1ull), t0, sub);
         }
         uint32_t flags = 0;
@@ -445,6 +452,10 @@ __global__ void __launch_bounds__(kThreads, 2) k_closure_persistent(PersistArgs 
             }
         }
         if (!go) break;
+        if (flags & kBarLeave) {
+            left = true;
+            break;
+        }
     }
 
     // ---- exit: clear the delta read in the last iteration; final state ----
@@ -489,7 +500,8 @@ __global__ void __launch_bounds__(kThreads, 2) k_closure_persistent(PersistArgs 
         st->items_by_variant[3] += m4r;
         st->last_changed = (uint32_t)(st->pbar[par] >> 32) & kBarChanged;
         st->iter = t + 1;
-        st->active = 0;
+        st->active = left ? 1u : 0u;
+        st->left = left ? 1u : 0u;
     }
     // the final state to the host without a copy after the kernel: the last
     // CTA past this point (every other CTA's statistics and block 0's final
@@ -539,9 +551,10 @@ cudaError_t launch_closure_persistent(int has_m4r, int grid, const ProdDesc *pro
                                       const SelectorParams *sel, SelLogRow *sel_log, uint32_t sel_log_iters,
                                       const QueryRange *qr, ItemTrace *trace, uint32_t *trace_count,
                                       int direct_merge, int prefetch, uint32_t spin_limit, int stall_barrier,
-                                      IterState *host_st, const uint32_t *flag_src, uint32_t *flag_dst,
-                                      cudaStream_t s) {
+                                      uint32_t leave_items, IterState *host_st, const uint32_t *flag_src,
+                                      uint32_t *flag_dst, cudaStream_t s) {
     PersistArgs a;
+    a.leave_idx = leave_items ? leave_items * (uint32_t)grid : kNoIndex;
     a.prods = prods;
     a.nprods = nprods;
     a.prod_rows = prod_rows;

@@ -61,11 +61,12 @@ __global__ void k_select(const ProdDesc *__restrict__ prods, uint32_t nprods, co
     }
 }
 
-// Buffer counters at closure start: current matrices from their occupancy
-// bitmaps and tile populations, deltas zero.  One block per slot.
+// Buffer counters of a closure from the occupancy bitmaps and tile
+// populations: block (slot, b), b = 0 the current matrix, 1 + d delta d.  Launched
+// with one block per slot, it takes the deltas as empty (closure start).
 __global__ void k_counters_init(const MatSlot *__restrict__ slots, BufCounters *cnts) {
-    const MatSlot sl = slots[blockIdx.x];
-    const DevMat m = sl.cur;
+    const uint32_t buf = blockIdx.y;
+    const DevMat m = buf ? slots[blockIdx.x].dlt[buf - 1] : slots[blockIdx.x].cur;
     unsigned long long nnz = 0;
     uint32_t occ = 0, dense = 0;
     const size_t tiles = (size_t)m.T * m.T, words = (size_t)m.T * m.ow;
@@ -96,9 +97,11 @@ __global__ void k_counters_init(const MatSlot *__restrict__ slots, BufCounters *
             c.occ_tiles += s_occ[w];
             c.dense_tiles += s_dense[w];
         }
-        cnts[3 * blockIdx.x] = c;
-        cnts[3 * blockIdx.x + 1] = BufCounters{0, 0, 0};
-        cnts[3 * blockIdx.x + 2] = BufCounters{0, 0, 0};
+        cnts[3 * blockIdx.x + buf] = c;
+        if (gridDim.y == 1) {
+            cnts[3 * blockIdx.x + 1] = BufCounters{0, 0, 0};
+            cnts[3 * blockIdx.x + 2] = BufCounters{0, 0, 0};
+        }
     }
 }
 
@@ -118,9 +121,10 @@ cudaError_t launch_select(const ProdDesc *d_prods, uint32_t nprods, const BufCou
     return cudaGetLastError();
 }
 
-cudaError_t launch_counters_init(const MatSlot *d_slots, uint32_t nslots, BufCounters *d_cnts, cudaStream_t s) {
+cudaError_t launch_counters_init(const MatSlot *d_slots, uint32_t nslots, BufCounters *d_cnts, bool with_deltas,
+                                 cudaStream_t s) {
     if (nslots == 0) return cudaSuccess;
-    k_counters_init<<<nslots, 256, 0, s>>>(d_slots, d_cnts);
+    k_counters_init<<<dim3(nslots, with_deltas ? 3 : 1), 256, 0, s>>>(d_slots, d_cnts);
     return cudaGetLastError();
 }
 

@@ -219,8 +219,11 @@ __global__ void __launch_bounds__(kThreads, 1)
         const uint64_t it = items[idx];
         const ProdDesc pd = prods[item_prod(it)];
         const uint32_t tig = item_ti(it), tjb = item_tjb(it), klo = item_klo(it), khi = item_khi(it);
-        const DevMat P = resolve_operand(slots[pd.pslot], pd.p_delta, iter);
-        const DevMat Q = resolve_operand(slots[pd.qslot], pd.q_delta, iter);
+        const bool merged = (it & kItemMerged) != 0;
+        const DevMat P = resolve_operand(slots[pd.pslot], merged ? 0 : pd.p_delta, iter);
+        const DevMat Q = resolve_operand(slots[pd.qslot], merged ? 0 : pd.q_delta, iter);
+        const uint32_t *const dpocc = slots[pd.pslot].dlt[iter & 1].occ;
+        const uint32_t *const dqocc = slots[pd.qslot].dlt[iter & 1].occ;
         const DevMat C = slots[pd.head].cur;
         const DevMat D = slots[pd.head].dlt[(iter & 1) ^ 1];
         const uint32_t T = pd.T, ow = P.ow;
@@ -259,7 +262,14 @@ __global__ void __launch_bounds__(kThreads, 1)
         for (uint32_t r = warp; r < rounds; r += kThreads / 32) {
             const uint32_t c = r * 32 + lane;
             uint32_t mask = 0;
-            if (c < nc) mask = (Q.occ[(size_t)S.cand[c] * ow + qword] >> qshift) & 0xFu;
+            if (c < nc) {
+                const uint32_t tk = S.cand[c];
+                bool dp = !merged;  // delta bits in the P tiles
+                if (merged)
+                    for (uint32_t g = 0; g < np; ++g)
+                        dp = dp || ((dpocc[(size_t)(ti0 + g) * ow + (tk >> 5)] >> (tk & 31)) & 1u);
+                mask = ((dp ? Q.occ : dqocc)[(size_t)tk * ow + qword] >> qshift) & 0xFu;
+            }
             const unsigned ball = __ballot_sync(kFull, mask != 0);
             if (c < nc) S.cmask[c] = (uint16_t)mask;
             if (lane == 0) S.rball[r] = ball;

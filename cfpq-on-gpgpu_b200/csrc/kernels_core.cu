@@ -413,8 +413,9 @@ __global__ void __launch_bounds__(kPlanThreads)
     __shared__ plan::WarpArea<plan::kPlanMaxBlocks> areas[kPlanThreads / 32];
     const uint32_t gw = row_begin + ((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
     if (gw >= total_rows || !st->active) return;
-    plan::plan_row(gw, prods, nprods, slots, st->iter, st, st->item_count, items_all, list_cap, tpb, prod_seen,
-                   tc_mode, ps, areas[threadIdx.x >> 5].cnt, areas[threadIdx.x >> 5].bnd);
+    plan::WarpArea<plan::kPlanMaxBlocks> &area = areas[threadIdx.x >> 5];
+    plan::plan_row<true>(gw, prods, nprods, slots, st->iter, st, st->item_count, items_all, list_cap, tpb, prod_seen,
+                   tc_mode, ps, area.cnt, area.bnd);
 }
 
 // Tensor-core plan of every tensor-core-capable product of a closure in one
@@ -434,8 +435,9 @@ __global__ void __launch_bounds__(kPlanThreads)
         if (tc[mid].pref <= r) lo = mid; else hi = mid;
     }
     const TcRows t = tc[lo];
-    plan::plan_row(t.row_start + (r - t.pref), prods, nprods, slots, st->iter, st, st->item_count, items_all,
-                   list_cap, tpb, prod_seen, 1, ps, areas[threadIdx.x >> 5].cnt, areas[threadIdx.x >> 5].bnd, t.prod,
+    plan::WarpArea<plan::kPlanMaxBlocks> &area = areas[threadIdx.x >> 5];
+    plan::plan_row<true>(t.row_start + (r - t.pref), prods, nprods, slots, st->iter, st, st->item_count, items_all,
+                   list_cap, tpb, prod_seen, 1, ps, area.cnt, area.bnd, t.prod,
                    t.prod + 1);
 }
 
@@ -703,7 +705,7 @@ cudaError_t launch_plan(const ProdDesc *d_prods, uint32_t nprods, uint32_t row_b
                         cudaStream_t s, const PlanSelect *sel, const uint32_t *d_q_last) {
     if (row_end <= row_begin || nprods == 0) return cudaSuccess;
     PlanSelect ps = sel ? *sel
-                        : PlanSelect{nullptr, nullptr, nullptr, const_cast<uint8_t *>(d_choice), nullptr, 0, nullptr};
+                        : PlanSelect{nullptr, nullptr, nullptr, const_cast<uint8_t *>(d_choice), nullptr, 0, nullptr, 0};
     ps.q_last = d_q_last;
     k_plan<<<grid_for((size_t)(row_end - row_begin) * 32, kPlanThreads), kPlanThreads, 0, s>>>(
         d_prods, nprods, row_begin, row_end, d_slots, d_st, d_items, list_cap, tiles_per_block, d_prod_seen, tc_mode,
@@ -716,7 +718,7 @@ cudaError_t launch_plan_tc(const ProdDesc *d_prods, uint32_t nprods, const TcRow
                            size_t list_cap, int tiles_per_block, uint32_t *d_prod_seen, const uint8_t *d_choice,
                            cudaStream_t s, const uint32_t *d_q_last) {
     if (ntc == 0 || total_groups == 0) return cudaSuccess;
-    const PlanSelect ps{nullptr, nullptr, nullptr, const_cast<uint8_t *>(d_choice), nullptr, 0, d_q_last};
+    const PlanSelect ps{nullptr, nullptr, nullptr, const_cast<uint8_t *>(d_choice), nullptr, 0, d_q_last, 0};
     k_plan_tc<<<grid_for((size_t)total_groups * 32, kPlanThreads), kPlanThreads, 0, s>>>(
         d_prods, nprods, d_tc, ntc, total_groups, d_slots, d_st, d_items, list_cap, tiles_per_block, d_prod_seen, ps);
     return cudaGetLastError();

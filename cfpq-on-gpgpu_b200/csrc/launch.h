@@ -145,8 +145,11 @@ cudaError_t launch_closure_persistent(int has_m4r, int grid, const ProdDesc *pro
                                       const SelectorParams *sel, SelLogRow *sel_log, uint32_t sel_log_iters,
                                       const QueryRange *qr, ItemTrace *trace, uint32_t *trace_count,
                                       int direct_merge, int prefetch, uint32_t spin_limit, int stall_barrier,
-                                      IterState *host_st, const uint32_t *flag_src, uint32_t *flag_dst,
-                                      cudaStream_t s);
+                                      uint32_t leave_items, IterState *host_st, const uint32_t *flag_src,
+                                      uint32_t *flag_dst, cudaStream_t s);
+// (leave_items non-zero: after an iteration with more work items per CTA the
+// kernel leaves with st->left set, st->active still 1 and the deltas as the
+// multi-kernel loop's next iteration expects them)
 // (spin_limit 0: the default of about a second of polling per wait;
 // trace non-null: one ItemTrace per processed item, counted in *trace_count)
 // (direct_merge: result words go to their atomic OR without reading C first)
@@ -161,8 +164,10 @@ cudaError_t launch_closure_persistent(int has_m4r, int grid, const ProdDesc *pro
 cudaError_t launch_select(const ProdDesc *d_prods, uint32_t nprods, const BufCounters *d_cnts, const IterState *d_st,
                           const SelectorParams *d_params, uint8_t *d_choice, const uint8_t *d_tc_ok,
                           SelLogRow *d_log, uint32_t log_iters, cudaStream_t s);
-// Buffer counters at closure start (current matrices measured, deltas zero).
-cudaError_t launch_counters_init(const MatSlot *d_slots, uint32_t nslots, BufCounters *d_cnts, cudaStream_t s);
+// Buffer counters of the current matrices; the deltas' too (with_deltas), else
+// zero (closure start).
+cudaError_t launch_counters_init(const MatSlot *d_slots, uint32_t nslots, BufCounters *d_cnts, bool with_deltas,
+                                 cudaStream_t s);
 cudaError_t launch_fill_choice(uint8_t *d_choice, uint32_t n, uint8_t v, cudaStream_t s);
 
 // Cost-model training and inference (kernel_mlp.cu); weights: kSelWeights floats.

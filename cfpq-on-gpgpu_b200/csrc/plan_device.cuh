@@ -45,7 +45,6 @@ __device__ __forceinline__ uint32_t nth_set_bit(uint32_t x, uint32_t n) {
 }
 
 constexpr uint32_t kPlanMaxBlocks = 512;  // T <= 2048 tiles, blocks of >= 4 tiles
-
 // Per-warp shared memory of the planner for up to kBlocks output blocks per
 // tile-row (512: any product; 128: word-level products, blocks of 16 tiles).
 template <uint32_t kBlocks>
@@ -60,6 +59,8 @@ struct WarpArea {
 // product statistics.  tc_mode 0 plans word-level products, 1 tensor-core ones.
 // unified_m4r non-null: every word-level item goes to list 0, Four Russians
 // items marked by bit 0 of the item and also counted in *unified_m4r.
+// kMerge false: the closure never merges rules (kItemMerged).
+template <bool kMerge>
 __device__ __forceinline__ void plan_row(uint32_t gw, const ProdDesc *__restrict__ prods, uint32_t nprods,
                                          const MatSlot *__restrict__ slots, uint32_t iter, IterState *st,
                                          uint32_t *item_count, uint64_t *__restrict__ items_all, size_t list_cap,
@@ -79,12 +80,17 @@ __device__ __forceinline__ void plan_row(uint32_t gw, const ProdDesc *__restrict
     if (pd.term == 1 && iter == 0) return;  // first iteration: delta(A) = A, one term covers A*B
     if (ps.q_last && iter > 0 && ps.q_last[pd.query] != iter) return;  // both terms read an empty delta
     uint32_t variant;  // this iteration's variant of the product
+    bool merged = false;
     if (ps.sel && !tc_mode) {
         float f[kSelFeatures], pred[kSelOutputs] = {0.f, 0.f, 0.f};
         uint32_t flags = 0;
-        variant = sel::select_product(pd, ps.cnts, iter, ps.sel, ps.tc_ok && ps.tc_ok[lo], f, pred, &flags);
+        merged = kMerge && ps.sel->mode != 0 && sel::merge_terms(pd, ps.cnts, iter, ps.static_counts != 0);
+        ProdDesc sd = pd;  // the operands the selection looks at
+        if (merged && pd.term == 0) sd.p_delta = 0;
+        variant = sel::select_product(sd, ps.cnts, iter, ps.sel, ps.tc_ok && ps.tc_ok[lo], f, pred, &flags);
+        if (merged && pd.term == 1) variant = 2;  // planned with the first term
         if (gw == pd.row_start && (threadIdx.x & 31) == 0) {
-            ps.choice[lo] = (uint8_t)variant;
+            ps.choice[lo] = (uint8_t)(variant | (merged && pd.term == 0 ? kChoiceMerged : 0u));
             if (ps.log && iter < ps.log_iters) {
                 SelLogRow &r = ps.log[(size_t)iter * nprods + lo];
                 for (int i = 0; i < kSelFeatures; ++i) r.f[i] = f[i];
@@ -92,20 +98,26 @@ __device__ __forceinline__ void plan_row(uint32_t gw, const ProdDesc *__restrict
                 r.choice = variant | flags;
             }
         }
+        if (merged && pd.term == 1) return;
     } else {
         variant = ps.choice ? ps.choice[lo] : pd.variant;
+        merged = kMerge && (variant & kChoiceMerged) != 0;
+        variant &= ~kChoiceMerged;
     }
     const bool tc = variant == 4;                                // CFPQ_VARIANT_TC
     if (tc != (tc_mode != 0)) return;  // word-level and tensor-core products are planned by separate launches
     const bool m4r = !tc && variant == 3;                        // CFPQ_VARIANT_M4R
     const uint32_t list = tc ? 2u : (m4r && !unified_m4r ? 1u : 0u);
-    const uint64_t vbit = m4r && unified_m4r ? 1u : 0u;
+    const uint64_t vbit = (m4r && unified_m4r ? kItemM4R : 0u) | (merged ? kItemMerged : 0u);
     if (tc) tpb = 4;
     const uint32_t rows_per_item = tc ? 4u : 1u;
     uint64_t *items = items_all + list * list_cap;
     const uint32_t ti = gw - pd.row_start;  // tile-row, or group of 4 tile-rows for tc
-    const DevMat P = resolve_operand(slots[pd.pslot], pd.p_delta, iter);
-    const DevMat Q = resolve_operand(slots[pd.qslot], pd.q_delta, iter);
+    const DevMat P = resolve_operand(slots[pd.pslot], merged ? 0 : pd.p_delta, iter);
+    const DevMat Q = resolve_operand(slots[pd.qslot], merged ? 0 : pd.q_delta, iter);
+    // merged: a k-tile whose P tile (row group) holds no bits of the delta
+    // counts only where its Q block does
+    const uint32_t *const dpocc = slots[pd.pslot].dlt[iter & 1].occ, *const dqocc = slots[pd.qslot].dlt[iter & 1].occ;
     const uint32_t T = pd.T, ow = P.ow;
     const uint32_t bpw = 32 / tpb;  // blocks per occupancy word
     const uint32_t bmask = tpb == 32 ? 0xffffffffu : ((1u << tpb) - 1);
@@ -115,6 +127,17 @@ __device__ __forceinline__ void plan_row(uint32_t gw, const ProdDesc *__restrict
         for (uint32_t g = 0; g < rows_per_item && ti * rows_per_item + g < T; ++g)
             bits |= P.occ[(size_t)(ti * rows_per_item + g) * ow + w];
         return bits;
+    };
+    auto delta_p = [&](uint32_t tk) {  // delta bits in P tile tk of the row (group)
+        uint32_t bits = 0;
+        for (uint32_t g = 0; g < rows_per_item && ti * rows_per_item + g < T; ++g)
+            bits |= dpocc[(size_t)(ti * rows_per_item + g) * ow + (tk >> 5)];
+        return ((bits >> (tk & 31)) & 1u) != 0;
+    };
+    // occupancy row of Q that the lane's candidate tk uses
+    auto q_row = [&](uint32_t tk, bool valid) {
+        const uint32_t *occ = merged && valid && !delta_p(tk) ? dqocc : Q.occ;
+        return occ + (size_t)tk * ow;
     };
     // occupied P tiles of the row (group); the first 32 occupancy words stay
     // in registers (one per lane) for the main loop
@@ -160,9 +183,9 @@ __device__ __forceinline__ void plan_row(uint32_t gw, const ProdDesc *__restrict
             const uint32_t bits = __shfl_sync(kFull, first, pw);  // 0 beyond ow
             const bool valid = lane < (uint32_t)__popc(bits);
             tks[pw] = valid ? pw * 32 + nth_set_bit(bits, lane) : 0u;
+            const uint32_t *qrow = q_row(tks[pw], valid);
 #pragma unroll
-            for (int u = 0; u < 4; ++u)
-                pre[pw][u] = (valid && (uint32_t)u < ow) ? Q.occ[(size_t)tks[pw] * ow + u] : 0u;
+            for (int u = 0; u < 4; ++u) pre[pw][u] = (valid && (uint32_t)u < ow) ? qrow[u] : 0u;
         }
 #pragma unroll
         for (int pw = 0; pw < 4; ++pw)
@@ -176,7 +199,7 @@ __device__ __forceinline__ void plan_row(uint32_t gw, const ProdDesc *__restrict
             if (!bits) continue;
             const bool valid = lane < (uint32_t)__popc(bits);
             const uint32_t tk = valid ? pw * 32 + nth_set_bit(bits, lane) : 0u;  // increasing with the lane
-            const uint32_t *qrow = Q.occ + (size_t)tk * ow;
+            const uint32_t *qrow = q_row(tk, valid);
             for (uint32_t w0 = 0; w0 < ow; w0 += 4) {
                 uint32_t m[4];
 #pragma unroll
@@ -196,7 +219,7 @@ __device__ __forceinline__ void plan_row(uint32_t gw, const ProdDesc *__restrict
     uint32_t pos0 = 0;
     if (lane == 0) {
         pos0 = atomicAdd(&item_count[list], total);
-        if (vbit) atomicAdd(unified_m4r, total);
+        if (m4r && unified_m4r) atomicAdd(unified_m4r, total);
     }
     pos0 = __shfl_sync(kFull, pos0, 0);
     for (uint32_t base = 0; base < nblocks; base += 32) {

@@ -85,9 +85,9 @@ struct ItemCounters {
 // straight to its atomic OR (one round trip less per item; for latency-bound
 // closures), else only words with bits C does not hold yet.  stamps non-null
 // (thread 0): %globaltimer after the k-list, after the first staged k-tile
-// arrived, after the last k-tile and after the gate.  Ends with the CTA
-// synchronised.
-template <bool kM4R, int kW, class Smem>
+// arrived, after the last k-tile and after the gate.  kMerge false: the
+// closure never merges rules (kItemMerged).  Ends with the CTA synchronised.
+template <bool kM4R, int kW, bool kMerge, class Smem>
 __device__ __forceinline__ void process_item(Smem &S, uint64_t it, const ProdDesc *__restrict__ prods,
                                              const MatSlot *__restrict__ slots, uint32_t iter, uint32_t *changed,
                                              uint32_t *qchanged, uint32_t &phase, bool &timed_out,
@@ -105,8 +105,10 @@ __device__ __forceinline__ void process_item(Smem &S, uint64_t it, const ProdDes
     unsigned long long &triples = ctr.triples, &staged = ctr.staged, &outw = ctr.outw, &neww = ctr.neww;
     const ProdDesc pd = prods[item_prod(it)];
     const uint32_t ti = item_ti(it), tjb = item_tjb(it), klo = item_klo(it), khi = item_khi(it);
-    const DevMat P = resolve_operand(slots[pd.pslot], pd.p_delta, iter);
-    const DevMat Q = resolve_operand(slots[pd.qslot], pd.q_delta, iter);
+    const bool merged = kMerge && (it & kItemMerged) != 0;
+    const DevMat P = resolve_operand(slots[pd.pslot], merged ? 0 : pd.p_delta, iter);
+    const DevMat Q = resolve_operand(slots[pd.qslot], merged ? 0 : pd.q_delta, iter);
+    const uint32_t *const dpocc = slots[pd.pslot].dlt[iter & 1].occ, *const dqocc = slots[pd.qslot].dlt[iter & 1].occ;
     const DevMat C = slots[pd.head].cur;
     const DevMat D = slots[pd.head].dlt[(iter & 1) ^ 1];
     const uint32_t T = pd.T, ow = P.ow;
@@ -127,7 +129,11 @@ __device__ __forceinline__ void process_item(Smem &S, uint64_t it, const ProdDes
         bool dense = false;
         if (tk < khi) {
             const uint32_t pw = P.occ[(size_t)ti * ow + (tk >> 5)];
-            const uint32_t qw = Q.occ[(size_t)tk * ow + qword];
+            uint32_t qw = Q.occ[(size_t)tk * ow + qword];
+            if (merged) {
+                const uint32_t dp = dpocc[(size_t)ti * ow + (tk >> 5)], dq = dqocc[(size_t)tk * ow + qword];
+                if (!((dp >> (tk & 31)) & 1u)) qw = dq;
+            }
             const uint32_t pn = P.nnz[(size_t)ti * T + tk];
             if ((pw >> (tk & 31)) & 1u) {
                 mask = (qw >> qshift) & ((1u << kBJ) - 1);
@@ -186,7 +192,8 @@ __device__ __forceinline__ void process_item(Smem &S, uint64_t it, const ProdDes
         bool dense = false;
         if (c < nc) {
             const uint32_t tk = S.cand[c];
-            mask = (Q.occ[(size_t)tk * ow + qword] >> qshift) & ((1u << kBJ) - 1);
+            const bool dp = !merged || ((dpocc[(size_t)ti * ow + (tk >> 5)] >> (tk & 31)) & 1u);
+            mask = ((dp ? Q.occ : dqocc)[(size_t)tk * ow + qword] >> qshift) & ((1u << kBJ) - 1);
             dense = P.nnz[(size_t)ti * T + tk] > kSparseMax;  // issued together with the occupancy load
         }
         const unsigned ball = __ballot_sync(kFull, mask != 0);
@@ -509,7 +516,7 @@ __device__ __forceinline__ void process_item(Smem &S, uint64_t it, const ProdDes
         if (D.bits) tiles_gain(D, ti, tj0 + kTPW * warp, mine, cnts ? cnts + 3 * pd.head + 1 + ((iter & 1) ^ 1) : nullptr);
     }
     if (any_new && lane == 0) {
-        *changed = 1u;
+        *reinterpret_cast<uint8_t *>(changed) = 1u;  // kBarChanged (the other bytes may carry other flags)
         if (qchanged) qchanged[pd.query] = 1u;
     }
     __syncthreads();  // k-list and stage reuse by the next item
