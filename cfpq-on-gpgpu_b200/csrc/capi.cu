@@ -61,6 +61,21 @@ constexpr uint32_t kPhaseLogIters = 4096;
 // on closures that are heavy only for a while (random CNF, grammar 5, n = 1800):
 // 1948, 1224, 1277, 1237 us; on dense ones (n = 900) 649, 656, 690, 817 us.
 constexpr uint32_t kLeaveItems = 12;
+// Largest tile counts of a single product that runs without a plan, on the
+// tensor cores or with the variant chosen on the device, and with a given
+// word-level variant.  Above them the empty work units of a sparse product
+// (one round trip each) outnumber the CTAs by too much: n = 12000 (188 tiles)
+// with 300 bits, Four Russians 54 us against 45 planned, LOP3 37 against 45;
+// dense LOP3 4631 against 4556.  At n = 8192: 30 against 36, 28 against 36, 1402 against
+// 1464.  AUTO at n = 12000 keeps the launch for its tensor cores: dense 1573 us
+// against 4556 with LOP3.
+constexpr uint32_t kAddMulMaxTiles = 256;
+constexpr uint32_t kAddMulMaxWordTiles = 128;
+// Slots of the context's pinned flag block that receive a single product's
+// changed and error words.
+constexpr int kAddMulSlot = 4;
+// First of the two work counters of a single product in the device flag block.
+constexpr int kAddMulWork = 8;
 // Iterations of a closure whose selection rows are kept.
 constexpr uint32_t kSelLogIters = 128;
 
@@ -263,6 +278,7 @@ extern "C" int cfpq_ctx_create(int device, cfpq_ctx **out) {
     for (auto &e : c->kev) CUDA_TRY(cudaEventCreate(&e));
     CUDA_TRY(cudaMalloc(&c->d_st, sizeof(IterState)));
     CUDA_TRY(cudaMalloc(&c->d_flag, 64));
+    CUDA_TRY(cudaMemset(c->d_flag, 0, 64));
     CUDA_TRY(cudaMalloc(&c->d_bad, 64));
     CUDA_TRY(cudaMallocHost(&c->h_st, sizeof(IterState)));
     CUDA_TRY(cudaMallocHost(&c->h_flag, 64));
@@ -897,6 +913,12 @@ static int add_mul_impl(cfpq_ctx *ctx, cfpq_matrix *c, const cfpq_matrix *a, con
         return set_error(CFPQ_ERR_INVALID, "operands have different vertex orders");
     *changed = 0;
     if (c->d.n == 0) return CFPQ_OK;
+    // AUTO: tensor cores or LOP3 by the selector's rule, decided on the device
+    // right before the product (choose, LOP3 and tensor-core launches, the one
+    // not chosen returns at once); below the tensor cores' size, LOP3
+    const bool choose = variant == CFPQ_VARIANT_AUTO && ctx->sel.mode != CFPQ_SELECT_FIXED && ctx->tc_grid &&
+                        (ctx->sel.allowed & (1u << CFPQ_VARIANT_TC)) && ctx->h_flag_dev &&
+                        c->d.T >= ctx->sel.tc_min_tiles && c->d.T <= kAddMulMaxTiles;
     if (variant == CFPQ_VARIANT_AUTO) variant = CFPQ_VARIANT_LOP3;
     const bool alias = (a == c) || (b == c);
     if (variant == CFPQ_VARIANT_PLAIN) {
@@ -932,6 +954,28 @@ static int add_mul_impl(cfpq_ctx *ctx, cfpq_matrix *c, const cfpq_matrix *a, con
             CUDA_TRY(launch_copy_matrix(cb->d, b->d, ctx->stream));
             db = cb->d;
         }
+    }
+    if (ctx->h_flag_dev &&
+        c->d.T <= (choose || variant == CFPQ_VARIANT_TC ? kAddMulMaxTiles : kAddMulMaxWordTiles)) {
+        uint32_t *const h_changed = ctx->h_flag + kAddMulSlot, *const h_error = h_changed + 1;
+        uint32_t *const d_changed = ctx->h_flag_dev + kAddMulSlot, *const d_error = d_changed + 1;
+        *h_changed = *h_error = 0;
+        uint32_t *const use_tc = choose ? ctx->d_flag : nullptr;
+        if (choose)
+            CUDA_TRY(launch_add_mul_choose(da, ctx->sel.tc_min_occ, ctx->sel.tc_min_dense, use_tc, ctx->stream));
+        if (variant != CFPQ_VARIANT_TC)
+            CUDA_TRY(launch_add_mul(variant == CFPQ_VARIANT_M4R, da, db, c->d, ti0, std::min(ti1, c->d.T),
+                                    variant == CFPQ_VARIANT_M4R ? ctx->m4r_grid : ctx->lop3_grid,
+                                    ctx->d_flag + kAddMulWork, use_tc, d_changed, d_error, ctx->stream));
+        if (variant == CFPQ_VARIANT_TC || choose)
+            CUDA_TRY(launch_add_mul_tc(da, db, c->d, ctx->tc_grid, use_tc, d_changed, d_error, ctx->stream));
+        CUDA_TRY(cudaStreamSynchronize(ctx->stream));
+        if (ca) TRY(pool_give(ctx, ca, true));
+        if (cb) TRY(pool_give(ctx, cb, true));
+        if (*(volatile uint32_t *)h_error)
+            return set_error(CFPQ_ERR_TIMEOUT, "a bounded device wait gave up (product kernel)");
+        *changed = *(volatile uint32_t *)h_changed != 0;
+        return CFPQ_OK;
     }
     TRY(enqueue_tiled_product(ctx, da, db, c->d, variant, ti0, ti1));
     CUDA_TRY(cudaMemcpyAsync(ctx->h_st, ctx->d_st, sizeof(IterState), cudaMemcpyDeviceToHost, ctx->stream));

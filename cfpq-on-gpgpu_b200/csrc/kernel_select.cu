@@ -105,6 +105,27 @@ __global__ void k_counters_init(const MatSlot *__restrict__ slots, BufCounters *
     }
 }
 
+// Variant of one product by itself (cfpq_add_mul with AUTO): the heuristic's
+// tensor-core rule on the left operand's tile statistics.  One block.
+__global__ void __launch_bounds__(1024) k_add_mul_choose(DevMat a, float min_occ, float min_dense, uint32_t *use_tc) {
+    const uint32_t tiles = a.T * a.T, words = a.T * a.ow;
+    uint32_t occ = 0, dense = 0;
+    for (uint32_t i = threadIdx.x; i < tiles; i += blockDim.x) dense += a.nnz[i] > kDenseTilePop;
+    for (uint32_t i = threadIdx.x; i < words; i += blockDim.x) occ += __popc(a.occ[i]);
+    occ = __reduce_add_sync(kFull, occ);
+    dense = __reduce_add_sync(kFull, dense);
+    __shared__ uint32_t s_occ, s_dense;
+    if (threadIdx.x == 0) s_occ = s_dense = 0;
+    __syncthreads();
+    if ((threadIdx.x & 31) == 0) {
+        atomicAdd(&s_occ, occ);
+        atomicAdd(&s_dense, dense);
+    }
+    __syncthreads();
+    if (threadIdx.x == 0)
+        *use_tc = s_occ && (float)s_occ >= min_occ * (float)tiles && (float)s_dense >= min_dense * (float)s_occ;
+}
+
 __global__ void k_fill_choice(uint8_t *choice, uint32_t n, uint8_t v) {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) choice[i] = v;
@@ -125,6 +146,11 @@ cudaError_t launch_counters_init(const MatSlot *d_slots, uint32_t nslots, BufCou
                                  cudaStream_t s) {
     if (nslots == 0) return cudaSuccess;
     k_counters_init<<<dim3(nslots, with_deltas ? 3 : 1), 256, 0, s>>>(d_slots, d_cnts);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_add_mul_choose(const DevMat &a, float min_occ, float min_dense, uint32_t *use_tc, cudaStream_t s) {
+    k_add_mul_choose<<<1, 1024, 0, s>>>(a, min_occ, min_dense, use_tc);
     return cudaGetLastError();
 }
 

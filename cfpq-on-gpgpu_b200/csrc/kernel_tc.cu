@@ -39,6 +39,8 @@
 // flag (which ends every other role's waits), the CTA then waits (bounded) for
 // each bulk copy and MMA still in flight, frees TMEM and reports
 // CFPQ_ERR_TIMEOUT.
+#include <algorithm>
+
 #include "launch.h"
 
 namespace cfpq {
@@ -167,9 +169,22 @@ __device__ __forceinline__ bool wait_or_abort(uint64_t *bar, uint32_t parity, co
     return false;
 }
 
+// The operands of one product by itself (cfpq_add_mul): the items are all
+// 4 x 4-tile blocks of C in order, dealt to the CTAs by number, and the
+// changed and error words go to mapped host memory -- no tables, plan or
+// state.
+struct TcSingle {
+    DevMat a, b, c;
+    const uint32_t *use_tc;  // non-null: nothing to do unless it is set
+    uint32_t *host_changed, *host_error;
+};
+
+template <bool kSingle>
 __global__ void __launch_bounds__(kThreads, 1)
     k_product_tc(const ProdDesc *__restrict__ prods, const MatSlot *__restrict__ slots, IterState *st,
-                 const uint64_t *__restrict__ items_all, size_t list_cap, uint32_t *qchanged, BufCounters *cnts) {
+                 const uint64_t *__restrict__ items_all, size_t list_cap, uint32_t *qchanged, BufCounters *cnts,
+                 TcSingle single) {
+    if (kSingle && single.use_tc && !*single.use_tc) return;
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     TcSmem &S = *reinterpret_cast<TcSmem *>(smem_raw);
     const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -200,8 +215,9 @@ __global__ void __launch_bounds__(kThreads, 1)
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = S.tmem_base;
-    const uint32_t iter = st->iter;
-    const uint32_t nitems = st->item_count[2];
+    const uint32_t iter = kSingle ? 0u : st->iter;
+    const uint32_t single_blocks = (single.a.T + 3) / 4;
+    const uint32_t nitems = kSingle ? single_blocks * single_blocks : st->item_count[2];
     unsigned long long triples = 0, outw = 0, neww = 0;
     // k-tile sequence numbers across the CTA's items: stage = seq % stages,
     // use = seq / stages; a "full" barrier is waited with parity use & 1, an
@@ -211,21 +227,31 @@ __global__ void __launch_bounds__(kThreads, 1)
     uint32_t pk_issued = 0;      // copy warp: packed stages issued (sequence count)
     uint32_t mma_committed = 0;  // MMA warp: k-tiles committed (sequence count)
 
-    for (;;) {
-        if (tid == 0) S.item = atomicAdd(&st->item_next[2], 1u);
-        __syncthreads();
-        const uint32_t idx = S.item;
+    bool single_changed = false;  // (kSingle) this thread saw a new bit
+    for (uint32_t round = 0;; ++round) {
+        if (!kSingle && tid == 0) S.item = atomicAdd(&st->item_next[2], 1u);
+        if (!kSingle) __syncthreads();
+        const uint32_t idx = kSingle ? blockIdx.x + round * gridDim.x : S.item;
         if (idx >= nitems || *abort) break;
-        const uint64_t it = items[idx];
-        const ProdDesc pd = prods[item_prod(it)];
+        const uint64_t it = kSingle ? make_item(0, idx / single_blocks, idx % single_blocks, 0, single.a.T) : items[idx];
+        ProdDesc pd;
+        if (kSingle) {
+            pd.T = single.a.T;
+            pd.query = 0;
+            pd.head = 0;
+        } else {
+            pd = prods[item_prod(it)];
+        }
         const uint32_t tig = item_ti(it), tjb = item_tjb(it), klo = item_klo(it), khi = item_khi(it);
-        const bool merged = (it & kItemMerged) != 0;
-        const DevMat P = resolve_operand(slots[pd.pslot], merged ? 0 : pd.p_delta, iter);
-        const DevMat Q = resolve_operand(slots[pd.qslot], merged ? 0 : pd.q_delta, iter);
-        const uint32_t *const dpocc = slots[pd.pslot].dlt[iter & 1].occ;
-        const uint32_t *const dqocc = slots[pd.qslot].dlt[iter & 1].occ;
-        const DevMat C = slots[pd.head].cur;
-        const DevMat D = slots[pd.head].dlt[(iter & 1) ^ 1];
+        const bool merged = !kSingle && (it & kItemMerged) != 0;
+        const DevMat P = kSingle ? single.a : resolve_operand(slots[pd.pslot], merged ? 0 : pd.p_delta, iter);
+        const DevMat Q = kSingle ? single.b : resolve_operand(slots[pd.qslot], merged ? 0 : pd.q_delta, iter);
+        const uint32_t *const dpocc = kSingle ? nullptr : slots[pd.pslot].dlt[iter & 1].occ;
+        const uint32_t *const dqocc = kSingle ? nullptr : slots[pd.qslot].dlt[iter & 1].occ;
+        const DevMat C = kSingle ? single.c : slots[pd.head].cur;
+        DevMat D;
+        if (kSingle) D.bits = nullptr;
+        else D = slots[pd.head].dlt[(iter & 1) ^ 1];
         const uint32_t T = pd.T, ow = P.ow;
         const uint32_t ti0 = tig * 4, tj0 = tjb * 4;
         const uint32_t qword = tj0 >> 5, qshift = tj0 & 31;
@@ -443,7 +469,9 @@ __global__ void __launch_bounds__(kThreads, 1)
             }
         }
         if (nk > 0) ++items_done;
-        if (any_new && lane == 0) {
+        if (kSingle) {
+            single_changed = single_changed || any_new;
+        } else if (any_new && lane == 0) {
             st->changed = 1u;
             if (qchanged) qchanged[pd.query] = 1u;
         }
@@ -471,17 +499,23 @@ __global__ void __launch_bounds__(kThreads, 1)
             mbar_wait_bounded(&S.op_empty[q % kOpStages], (q / kOpStages) & 1u);
         }
     }
-    for (int o = 16; o > 0; o >>= 1) {
-        triples += __shfl_down_sync(kFull, triples, o);
-        outw += __shfl_down_sync(kFull, outw, o);
-        neww += __shfl_down_sync(kFull, neww, o);
+    if (kSingle) {
+        const bool changed = __syncthreads_or(single_changed) != 0;
+        if (changed && tid == 0) *single.host_changed = 1u;
+        if (aborted && tid == 0) *single.host_error = 5u;
+    } else {
+        for (int o = 16; o > 0; o >>= 1) {
+            triples += __shfl_down_sync(kFull, triples, o);
+            outw += __shfl_down_sync(kFull, outw, o);
+            neww += __shfl_down_sync(kFull, neww, o);
+        }
+        if (lane == 0) {
+            if (triples) atomicAdd(&st->tile_triples, triples);
+            if (outw) atomicAdd(&st->out_words, outw);
+            if (neww) atomicAdd(&st->new_words, neww);
+        }
+        if (aborted && tid == 0) atomicExch(&st->error, 5u);
     }
-    if (lane == 0) {
-        if (triples) atomicAdd(&st->tile_triples, triples);
-        if (outw) atomicAdd(&st->out_words, outw);
-        if (neww) atomicAdd(&st->new_words, neww);
-    }
-    if (aborted && tid == 0) atomicExch(&st->error, 5u);
     tc_fence_before();
     __syncthreads();
     if (warp == 0)
@@ -491,16 +525,28 @@ __global__ void __launch_bounds__(kThreads, 1)
 }  // namespace
 
 int product_tc_blocks_per_sm() {
-    cudaFuncSetAttribute(k_product_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(TcSmem));
-    int nb = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_product_tc, kThreads, sizeof(TcSmem));
-    return nb;
+    cudaFuncSetAttribute(k_product_tc<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(TcSmem));
+    cudaFuncSetAttribute(k_product_tc<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(TcSmem));
+    int nb = 0, nb1 = 0;
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_product_tc<false>, kThreads, sizeof(TcSmem));
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb1, k_product_tc<true>, kThreads, sizeof(TcSmem));
+    return nb == nb1 ? nb : 0;
 }
 
 cudaError_t launch_product_tc(const ProdDesc *d_prods, const MatSlot *d_slots, IterState *d_st,
                               const uint64_t *d_items, size_t list_cap, uint32_t *d_qchanged, int grid,
                               BufCounters *cnts, cudaStream_t s) {
-    k_product_tc<<<grid, kThreads, sizeof(TcSmem), s>>>(d_prods, d_slots, d_st, d_items, list_cap, d_qchanged, cnts);
+    k_product_tc<false><<<grid, kThreads, sizeof(TcSmem), s>>>(d_prods, d_slots, d_st, d_items, list_cap, d_qchanged,
+                                                               cnts, TcSingle{});
+    return cudaGetLastError();
+}
+
+cudaError_t launch_add_mul_tc(const DevMat &a, const DevMat &b, const DevMat &c, int grid, const uint32_t *use_tc,
+                              uint32_t *host_changed, uint32_t *host_error, cudaStream_t s) {
+    if (a.T == 0) return cudaSuccess;
+    const uint32_t blocks = (a.T + 3) / 4;
+    k_product_tc<true><<<std::min((uint32_t)grid, blocks * blocks), kThreads, sizeof(TcSmem), s>>>(
+        nullptr, nullptr, nullptr, nullptr, 0, nullptr, nullptr, TcSingle{a, b, c, use_tc, host_changed, host_error});
     return cudaGetLastError();
 }
 

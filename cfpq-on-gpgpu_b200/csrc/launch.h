@@ -103,6 +103,23 @@ cudaError_t launch_product_tc(const ProdDesc *d_prods, const MatSlot *d_slots, I
 int product_tc_blocks_per_sm();
 // Closes a tensor-core product's item list (counts it, resets the counters).
 cudaError_t launch_reset_list(IterState *st, int list, cudaStream_t s);
+// One product c |= a * b on the tile-rows [ti0, ti1) (operands must not alias
+// c) in one launch, word-level; *host_changed = 1 if a bit of c changed,
+// *host_error = 5 if a bounded wait gave up (mapped host words, zeroed by the
+// caller).  grid: the resident CTAs of the variant's product kernel.  work: two device words, 0 before the first launch (every launch
+// leaves them 0).
+cudaError_t launch_add_mul(int m4r, const DevMat &a, const DevMat &b, const DevMat &c, uint32_t ti0, uint32_t ti1,
+                           int grid, uint32_t *work, const uint32_t *use_tc, uint32_t *host_changed,
+                           uint32_t *host_error, cudaStream_t s);
+// The same on the tensor cores (every tile-row).  use_tc (both; may be null):
+// device word of launch_add_mul_choose -- the word-level launch does nothing
+// when it is set, the tensor-core launch nothing when it is not.
+cudaError_t launch_add_mul_tc(const DevMat &a, const DevMat &b, const DevMat &c, int grid, const uint32_t *use_tc,
+                              uint32_t *host_changed, uint32_t *host_error, cudaStream_t s);
+// *use_tc = whether the tensor cores should run a product with left operand a
+// (the selector's rule: occupied-tile fraction >= min_occ, dense share of the
+// occupied tiles >= min_dense).
+cudaError_t launch_add_mul_choose(const DevMat &a, float min_occ, float min_dense, uint32_t *use_tc, cudaStream_t s);
 int product_lop3_tiles_per_block();
 int product_lop3_max_tiles();
 // Called once per context before any capture: sets kernel attributes, returns
