@@ -76,6 +76,14 @@ constexpr uint32_t kAddMulMaxWordTiles = 128;
 constexpr int kAddMulSlot = 4;
 // First of the two work counters of a single product in the device flag block.
 constexpr int kAddMulWork = 8;
+// Rows per CTA and iteration above which a closure of T tiles leaves the cluster
+// kernel for the persistent one, whose iterations cost 10-27 us at these sizes:
+// a cluster iteration of 1656 rows takes 8.5 us (brackets, n = 300), 2868 rows 26
+// us (n = 1024), 2709 rows 26 us (random CNF, n = 1000); but with the rows on few
+// warps 2180 take 65 us (dense random CNF, n = 260), and the next iteration of
+// such a closure reads 17 times as many.  With 16384 for every size that closure
+// takes 414 us instead of 353, one at n = 600 912 instead of 628.
+static inline uint32_t leave_reads(uint32_t T) { return 1024 + 128 * T; }
 // Iterations of a closure whose selection rows are kept.
 constexpr uint32_t kSelLogIters = 128;
 
@@ -298,6 +306,7 @@ extern "C" int cfpq_ctx_create(int device, cfpq_ctx **out) {
     int coop = 0;
     cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, device);
     for (int m = 0; m < 2; ++m) c->persist_grid[m] = coop ? persistent_blocks_per_sm(m) * c->num_sms : 0;
+    c->cluster_ok = cluster_closure_available() != 0;
     selector_defaults(&c->sel);
     if (!c->tc_grid) c->sel.allowed &= ~(1u << CFPQ_VARIANT_TC);
     *out = c;
@@ -722,7 +731,9 @@ static int ensure_hash_buffers(cfpq_ctx *ctx, size_t nm, size_t blocks) {
 // Hash launches of several matrices (one kernel per kHashBatch matrices, one
 // block per tile-row); their (hash, count) pairs land in the pinned h_hash
 // with no copy after the kernel when h_hash is mapped.
-static int enqueue_hash_many(cfpq_ctx *ctx, cfpq_matrix *const *mats, size_t nmats) {
+// skip_if_set (may be null): a device word that turns the launches into no-ops.
+static int enqueue_hash_many(cfpq_ctx *ctx, cfpq_matrix *const *mats, size_t nmats,
+                             const uint32_t *skip_if_set = nullptr) {
     size_t blocks = 0;
     for (size_t i0 = 0; i0 < nmats; i0 += kHashBatch) {
         size_t b = 0;
@@ -752,7 +763,7 @@ static int enqueue_hash_many(cfpq_ctx *ctx, cfpq_matrix *const *mats, size_t nma
                                           ctx->stream));
             continue;
         }
-        CUDA_TRY(launch_hash_lines(hb, ctx->d_hash_part, ctx->d_hash_ticket, out + 2 * i0, ctx->stream));
+        CUDA_TRY(launch_hash_lines(hb, ctx->d_hash_part, ctx->d_hash_ticket, out + 2 * i0, skip_if_set, ctx->stream));
     }
     if (!ctx->h_hash_dev)
         CUDA_TRY(cudaMemcpyAsync(ctx->h_hash, ctx->d_hash, nmats * 2 * sizeof(unsigned long long),
@@ -1573,6 +1584,25 @@ static void fill_hash_out(const cfpq_ctx *ctx, const HashOut *ho) {
     }
 }
 
+// The query's rules sorted by head, for the cluster kernel.
+static ClusterRules cluster_rules(const QueryIn &q) {
+    ClusterRules r;
+    memset(&r, 0, sizeof(r));
+    for (uint32_t head = 0; head < q.nmats; ++head) {
+        const uint32_t first = r.nrules;
+        for (size_t i = 0; i < q.nrules; ++i)
+            if (q.rules[i].head == head) {
+                r.body1[r.nrules] = (uint8_t)q.rules[i].body1;
+                r.body2[r.nrules++] = (uint8_t)q.rules[i].body2;
+            }
+        if (r.nrules == first) continue;
+        r.head[r.nheads] = (uint8_t)head;
+        r.start[r.nheads++] = (uint8_t)first;
+        r.start[r.nheads] = (uint8_t)r.nrules;
+    }
+    return r;
+}
+
 // Second stage of a late-selecting closure (ClosurePlan::late_select) whose
 // iterations became heavy: the persistent kernel has left after iteration
 // st->iter - 1 with the deltas ready for the next one; the counters are
@@ -1659,6 +1689,9 @@ static int run_engine(cfpq_ctx *ctx, const std::vector<QueryIn> &qs, const cfpq_
     const int persist_grid = ctx->persist_grid[pl.uses_m4r ? 1 : 0];
     const bool persistent =
         o.use_graph == CFPQ_LOOP_DEVICE && !timed && !log_products && !pl.uses_tc && persist_grid > 0;
+    // a small query starts inside one cluster's shared memory
+    const bool small = persistent && pl.late_select && nq == 1 && ctx->cluster_ok && !o.log_products && !o.wait_limit &&
+                       !o.test_flags && cluster_closure_fits((uint32_t)qs[0].nmats, qs[0].nrules, pl.prods[0].n);
     const uint32_t nprods = (uint32_t)pl.prods.size(), nslots = (uint32_t)pl.slots.size();
     TRY(ctx->items.ensure((persistent ? 4 : 3) * pl.item_cap * 8));
     // the persistent kernel's item lists: zero entries mean "not yet written";
@@ -1743,19 +1776,8 @@ static int run_engine(cfpq_ctx *ctx, const std::vector<QueryIn> &qs, const cfpq_
     if (o.use_graph && !timed && !log_products && !persistent) TRY(get_loop_graph(ctx, pl, qt, &exec));
     if (timed) memset(&ctx->prof, 0, sizeof(ctx->prof));
 
-    CUDA_TRY(cudaEventRecord(ctx->ev0, ctx->stream));
-    if (log_products) {
-        TRY(run_logged_iterations(ctx, pl, qt));
-    } else if (timed) {
-        for (uint32_t it = 0;; ++it) {
-            TRY(enqueue_iteration_timed(ctx, pl, qt));
-            CUDA_TRY(cudaMemcpyAsync(ctx->h_st, ctx->d_st, sizeof(IterState), cudaMemcpyDeviceToHost, ctx->stream));
-            CUDA_TRY(cudaStreamSynchronize(ctx->stream));
-            TRY(accumulate_kernel_times(ctx));
-            if (!ctx->h_st->active) break;
-            if (it > (1u << 24)) return set_error(CFPQ_ERR_CUDA, "closure did not converge");
-        }
-    } else if (persistent) {
+    // the persistent kernel, from iteration st->iter on
+    auto run_persistent = [&]() -> int {
         CUDA_TRY(launch_closure_persistent(pl.uses_m4r ? 1 : 0, persist_grid, ctx->prods.as<ProdDesc>(),
                                            (uint32_t)pl.prods.size(), pl.prod_rows, ctx->slots.as<MatSlot>(),
                                            (uint32_t)pl.slots.size(), pl.slot_rows, ctx->d_st,
@@ -1781,6 +1803,30 @@ static int run_engine(cfpq_ctx *ctx, const std::vector<QueryIn> &qs, const cfpq_
                                            flag_mapped ? ho->flag_src : nullptr,
                                            flag_mapped ? ctx->h_flag_dev + (ho->flag_dst - ctx->h_flag) : nullptr,
                                            ctx->stream));
+        return CFPQ_OK;
+    };
+    CUDA_TRY(cudaEventRecord(ctx->ev0, ctx->stream));
+    if (log_products) {
+        TRY(run_logged_iterations(ctx, pl, qt));
+    } else if (timed) {
+        for (uint32_t it = 0;; ++it) {
+            TRY(enqueue_iteration_timed(ctx, pl, qt));
+            CUDA_TRY(cudaMemcpyAsync(ctx->h_st, ctx->d_st, sizeof(IterState), cudaMemcpyDeviceToHost, ctx->stream));
+            CUDA_TRY(cudaStreamSynchronize(ctx->stream));
+            TRY(accumulate_kernel_times(ctx));
+            if (!ctx->h_st->active) break;
+            if (it > (1u << 24)) return set_error(CFPQ_ERR_CUDA, "closure did not converge");
+        }
+    } else if (persistent) {
+        if (small)
+            CUDA_TRY(launch_closure_cluster(ctx->slots.as<MatSlot>(), nslots, pl.prods[0].n, cluster_rules(qs[0]),
+                                            ctx->d_st, qt, ctx->phase_log.as<unsigned long long>(), kPhaseLogIters,
+                                            leave_reads(pl.prods[0].T), st_mapped ? ctx->h_st_dev : nullptr,
+                                            flag_mapped ? ho->flag_src : nullptr,
+                                            flag_mapped ? ctx->h_flag_dev + (ho->flag_dst - ctx->h_flag) : nullptr,
+                                            ctx->stream));
+        else
+            TRY(run_persistent());
     } else if (exec) {
         CUDA_TRY(cudaGraphLaunch(exec, ctx->stream));
     } else {
@@ -1821,12 +1867,23 @@ static int run_engine(cfpq_ctx *ctx, const std::vector<QueryIn> &qs, const cfpq_
         CUDA_TRY(cudaMemcpyAsync(h_done, qt.done_ns, nq * 8, cudaMemcpyDeviceToHost, ctx->stream));
         CUDA_TRY(cudaMemcpyAsync(h_last, qt.last_iter, nq * 4, cudaMemcpyDeviceToHost, ctx->stream));
     }
-    if (ho && ho->n) TRY(enqueue_hash_many(ctx, ho->mats, ho->n));
+    // (a closure that left its kernel before the fixpoint is hashed when it is done)
+    if (ho && ho->n) TRY(enqueue_hash_many(ctx, ho->mats, ho->n, pl.late_select ? &ctx->d_st->active : nullptr));
     if (ho && ho->flag_src && !flag_mapped)
         CUDA_TRY(cudaMemcpyAsync(ho->flag_dst, ho->flag_src, 4, cudaMemcpyDeviceToHost, ctx->stream));
     CUDA_TRY(cudaStreamSynchronize(ctx->stream));
     const IterState &hs = *ctx->h_st;
-    ctx->phase_log_iters = persistent ? std::min<uint32_t>(hs.iter, kPhaseLogIters) : 0;
+    const uint32_t cluster_iters = small ? hs.iter : 0;
+    const bool moved = small && hs.left;  // the cluster kernel left: on with the persistent kernel
+    if (moved) {
+        TRY(run_persistent());
+        CUDA_TRY(cudaEventRecord(ctx->ev1, ctx->stream));
+        if (!st_mapped)
+            CUDA_TRY(cudaMemcpyAsync(ctx->h_st, ctx->d_st, sizeof(IterState), cudaMemcpyDeviceToHost, ctx->stream));
+        if (ho && ho->n) TRY(enqueue_hash_many(ctx, ho->mats, ho->n, &ctx->d_st->active));
+        CUDA_TRY(cudaStreamSynchronize(ctx->stream));
+    }
+    ctx->phase_log_iters = persistent ? std::min<uint32_t>(hs.iter - (moved ? cluster_iters : 0), kPhaseLogIters) : 0;
     const uint32_t persistent_iters = persistent ? hs.iter : 0;
     const bool left = persistent && hs.left && !hs.error;
     if (left) TRY(finish_selected(ctx, pl, qt, nslots, ho));
@@ -1856,8 +1913,8 @@ static int run_engine(cfpq_ctx *ctx, const std::vector<QueryIn> &qs, const cfpq_
         const uint64_t input_launches = input ? 1 + (input->nedges ? 1 : 0) + (input->ndiag ? 1 : 0) : 0;
         stats->kernel_launches = input_launches + (ctx->cnts_on ? 1 : 0) + (input ? 0 : 1) +
                                  (persistent ? 1 + (uint64_t)(hs.iter - persistent_iters) * 3 : (uint64_t)hs.iter * 3) +
-                                 (ho && ho->n ? (ho->n + kHashBatch - 1) / kHashBatch * (left ? 2 : 1) : 0) +
-                                 (left ? 1 : 0);
+                                 (ho && ho->n ? (ho->n + kHashBatch - 1) / kHashBatch * (1 + left + moved) : 0) +
+                                 (left ? 1 : 0) + (moved ? 1 : 0);
         stats->variant_items[CFPQ_VARIANT_LOP3] = hs.items_by_variant[2];
         stats->variant_items[CFPQ_VARIANT_M4R] = hs.items_by_variant[3];
         stats->variant_items[CFPQ_VARIANT_TC] = hs.items_by_variant[4];

@@ -135,6 +135,7 @@ struct cfpq_ctx {
     uint64_t plan_ids = 0;
     uint64_t tables_owner = 0;  // plan id whose slot / product tables are in `slots` / `prods`
     int lop3_grid = 0, m4r_grid = 0, tc_grid = 0;  // tc_grid 0: tensor-core variant unavailable
+    bool cluster_ok = false;       // small closures may run in one thread-block cluster
     int persist_grid[2] = {0, 0};  // persistent closure CTAs [with M4R items]; 0: unavailable
     DevBuf phase_log;              // persistent closure: 3 timestamps per iteration
     DevBuf qranges;                // persistent closure of a batch: QueryRange per query

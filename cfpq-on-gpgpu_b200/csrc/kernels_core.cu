@@ -289,7 +289,9 @@ __device__ __forceinline__ void block_sum2(unsigned long long &h, unsigned long 
 // (< 2^30) before they are added up, and a matrix has fewer than 2^26
 // tile-rows.
 __global__ void __launch_bounds__(256, 6) k_hash_lines(HashBatch hb, unsigned long long *__restrict__ partial,
-                                                       uint32_t *ticket, unsigned long long *out) {
+                                                       uint32_t *ticket, unsigned long long *out,
+                                                       const uint32_t *skip) {
+    const uint32_t skipped = skip ? __ldcg(skip) : 0u;  // looked at when the row is summed: not a round trip more
     const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
     uint32_t i = 0;
     while (i + 1 < hb.count && blockIdx.x >= hb.start[i + 1]) ++i;
@@ -315,6 +317,7 @@ __global__ void __launch_bounds__(256, 6) k_hash_lines(HashBatch hb, unsigned lo
         }
     }
     unsigned long long h = (acc0 % kHashMod) * q0 % kHashMod + (acc1 % kHashMod) * q1 % kHashMod;
+    if (skipped) return;
     block_sum2(h, cnt);
     __shared__ bool last;
     if (threadIdx.x == 0) {
@@ -726,9 +729,9 @@ cudaError_t launch_pow_nibbles(const uint32_t *d_pow11, uint32_t T, uint32_t *d_
 }
 
 cudaError_t launch_hash_lines(const HashBatch &hb, unsigned long long *d_partial, uint32_t *d_ticket,
-                              unsigned long long *out, cudaStream_t s) {
+                              unsigned long long *out, const uint32_t *d_skip, cudaStream_t s) {
     if (hb.count == 0 || hb.start[hb.count] == 0) return cudaErrorInvalidValue;
-    k_hash_lines<<<hb.start[hb.count], 256, 0, s>>>(hb, d_partial, d_ticket, out);
+    k_hash_lines<<<hb.start[hb.count], 256, 0, s>>>(hb, d_partial, d_ticket, out, d_skip);
     return cudaGetLastError();
 }
 

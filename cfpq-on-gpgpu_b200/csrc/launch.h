@@ -49,7 +49,8 @@ cudaError_t launch_clear_rows(const MatRows *d_tab, uint32_t nmats, uint32_t tot
 // blocks [start[i], start[i+1])), partial sums in d_partial (2 words per
 // block), and the last block writes out[2i] = hash, out[2i+1] = bit count.
 // d_ticket must be 0 before the first launch (every launch leaves it 0);
-// out may be mapped host memory.  start[count] must be > 0.
+// out may be mapped host memory.  start[count] must be > 0.  d_skip (may be
+// null): nothing is done, out untouched, when this device word is set.
 constexpr uint32_t kHashBatch = 16;
 struct HashBatch {
     DevMat m[kHashBatch];
@@ -59,7 +60,7 @@ struct HashBatch {
     uint32_t count;
 };
 cudaError_t launch_hash_lines(const HashBatch &hb, unsigned long long *d_partial, uint32_t *d_ticket,
-                              unsigned long long *out, cudaStream_t s);
+                              unsigned long long *out, const uint32_t *d_skip, cudaStream_t s);
 // sub[tj * 256 + p * 16 + v] = sum over the set bits b of v of pow11[64 tj + 4 p + b]
 // (mod 1e9+7) for the T tile columns: a row's column term is the sum of 16
 // entries, one per nibble of its tile word.
@@ -150,6 +151,22 @@ cudaError_t launch_closure_begin(const ClosureBegin &a, int num_sms, cudaStream_
 // scatter, diagonals.
 cudaError_t launch_closure_input(const ClosureInput &in, int num_sms, cudaStream_t s,
                                  const ClosureBegin *begin = nullptr);
+// Small closure in one thread-block cluster (kernel_cluster.cu): queries of at
+// most 1024 vertices whose matrices and deltas fit the cluster's shared memory.
+// Rules sorted by head: head[i]'s rules are start[i] .. start[i + 1].
+struct ClusterRules {
+    static constexpr uint32_t kMats = 32, kRules = 64;
+    uint32_t nheads, nrules;
+    uint8_t head[kMats], start[kMats + 1], body1[kRules], body2[kRules];
+};
+int cluster_closure_available();  // sets the kernels' attributes; 0: the device cannot hold such a cluster
+bool cluster_closure_fits(uint32_t nmats, size_t nrules, uint32_t n);
+// Leaves before the fixpoint (st->left, as launch_closure_persistent) when the
+// next iteration would read more than leave_reads rows per CTA.
+cudaError_t launch_closure_cluster(const MatSlot *slots, uint32_t nmats, uint32_t n, const ClusterRules &rules,
+                                   IterState *st, const QueryTrack &qt, unsigned long long *phase_log,
+                                   uint32_t phase_log_iters, uint32_t leave_reads, IterState *host_st,
+                                   const uint32_t *flag_src, uint32_t *flag_dst, cudaStream_t s);
 // Persistent closure (word-level variants only): the whole fixpoint in one
 // cooperative launch of `grid` CTAs (at most persistent_blocks_per_sm() per
 // SM); items: 4 lists of list_cap; phase_log: 3 timestamps per iteration.
