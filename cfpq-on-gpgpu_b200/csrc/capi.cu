@@ -74,6 +74,8 @@ constexpr uint32_t kAddMulMaxWordTiles = 128;
 // Slots of the context's pinned flag block that receive a single product's
 // changed and error words.
 constexpr int kAddMulSlot = 4;
+// Slot that tells cfpq_load_edges of ids out of range.
+constexpr int kLoadBadSlot = 6;
 // First of the two work counters of a single product in the device flag block.
 constexpr int kAddMulWork = 8;
 // Rows per CTA and iteration above which a closure of T tiles leaves the cluster
@@ -288,6 +290,7 @@ extern "C" int cfpq_ctx_create(int device, cfpq_ctx **out) {
     CUDA_TRY(cudaMalloc(&c->d_flag, 64));
     CUDA_TRY(cudaMemset(c->d_flag, 0, 64));
     CUDA_TRY(cudaMalloc(&c->d_bad, 64));
+    CUDA_TRY(cudaMemset(c->d_bad, 0, 64));
     CUDA_TRY(cudaMallocHost(&c->h_st, sizeof(IterState)));
     CUDA_TRY(cudaMallocHost(&c->h_flag, 64));
     // the persistent kernel writes its final state straight into these
@@ -346,6 +349,7 @@ extern "C" int cfpq_ctx_destroy(cfpq_ctx *ctx) {
     if (ctx->h_hash) cudaFreeHost(ctx->h_hash);
     if (ctx->h_small) cudaFreeHost(ctx->h_small);
     if (ctx->h_query) cudaFreeHost(ctx->h_query);
+    if (ctx->h_edges) cudaFreeHost(ctx->h_edges);
     cudaEventDestroy(ctx->ev0);
     cudaEventDestroy(ctx->ev1);
     for (auto &e : ctx->kev) cudaEventDestroy(e);
@@ -445,8 +449,7 @@ static int load_edges_impl(cfpq_ctx *ctx, cfpq_matrix *const *mats, size_t nmats
 extern "C" int cfpq_load_edges(cfpq_ctx *ctx, cfpq_matrix *const *mats, size_t nmats, const uint32_t *from,
                                const uint32_t *label, const uint32_t *to, size_t nedges,
                                const uint32_t *label_offsets, const uint32_t *label_mats, uint32_t nlabels) {
-    TRY(load_edges_impl(ctx, mats, nmats, from, label, to, nedges, label_offsets, label_mats, nlabels, false));
-    return check_bad(ctx, "cfpq_load_edges");
+    return load_edges_impl(ctx, mats, nmats, from, label, to, nedges, label_offsets, label_mats, nlabels, false);
 }
 
 extern "C" int cfpq_load_edges_device(cfpq_ctx *ctx, cfpq_matrix *const *mats, size_t nmats, const uint32_t *d_from,
@@ -475,13 +478,33 @@ static const uint32_t *mapped_host_array(const uint32_t *a, size_t n) {
     return dev[1] == dev[0] + (n - 1) ? dev[0] : nullptr;
 }
 
+// The pinned block that short pageable edge lists are copied into, mapped on the
+// device; false if there is none.
+constexpr size_t kEdgeStageBytes = 256 << 10;
+static bool ensure_edge_stage(cfpq_ctx *ctx) {
+    if (ctx->h_edges) return ctx->h_edges_dev != nullptr;
+    if (cudaMallocHost(&ctx->h_edges, kEdgeStageBytes) != cudaSuccess) {
+        ctx->h_edges = nullptr;
+        cudaGetLastError();
+        return false;
+    }
+    if (cudaHostGetDevicePointer(reinterpret_cast<void **>(&ctx->h_edges_dev), ctx->h_edges, 0) != cudaSuccess) {
+        ctx->h_edges_dev = nullptr;
+        cudaGetLastError();
+    }
+    return ctx->h_edges_dev != nullptr;
+}
+
 // Validates an edge list and stages it for the scatter: the small tables
-// (matrix descriptors, label offsets, label -> matrices) on the device, host
-// edge arrays copied (asynchronously) into the context's staging block --
-// except with read_pinned_in_place, where arrays in pinned mapped host
-// memory are read by the scatter kernel itself over the bus (the caller must
-// keep them unchanged until the stream has run the kernel; *read_in_place
-// tells which happened).  Fills the edge fields of *in; launches nothing.
+// (matrix descriptors, label offsets, label -> matrices) for the scatter's
+// arguments (large ones on the device), host edge arrays copied
+// (asynchronously) into the context's staging block -- except with
+// read_pinned_in_place: the caller synchronises before it returns or anything
+// else overwrites the edges, so arrays in pinned mapped host memory are read
+// by the scatter kernel itself over the bus, and short pageable ones (up to
+// kEdgeStageBytes) from a pinned block they are copied into, which saves three
+// stream copies of 5-8 us each (*read_in_place tells that the kernel reads
+// host memory).  Fills the edge fields of *in; launches nothing.
 // Nothing to scatter: in->nedges = 0.
 static int prepare_edges(cfpq_ctx *ctx, cfpq_matrix *const *mats, size_t nmats, const uint32_t *from,
                          const uint32_t *label, const uint32_t *to, size_t nedges, const uint32_t *label_offsets,
@@ -503,62 +526,94 @@ static int prepare_edges(cfpq_ctx *ctx, cfpq_matrix *const *mats, size_t nmats, 
     }
     for (uint32_t j = 0; j < nlm; ++j)
         if (label_mats[j] >= nmats) return set_error(CFPQ_ERR_INVALID, "label_mats[%u] out of range", j);
-    // one staging block: descs | from | label | to | offsets | label_mats
     const size_t bd = nmats * sizeof(DevMat);
     const size_t be = nedges * 4;
     const size_t bo = (size_t)(nlabels + 1) * 4;
     const size_t bl = (size_t)(nlm ? nlm : 1) * 4;
-    auto up = [](size_t x) { return (x + 255) & ~(size_t)255; };
-    TRY(ctx->edge_buf.ensure(up(bd) + 3 * up(be) + up(bo) + up(bl)));
-    char *base = ctx->edge_buf.as<char>();
-    DevMat *d_desc = reinterpret_cast<DevMat *>(base);
-    uint32_t *d_from = reinterpret_cast<uint32_t *>(base + up(bd));
-    uint32_t *d_label = reinterpret_cast<uint32_t *>(base + up(bd) + up(be));
-    uint32_t *d_to = reinterpret_cast<uint32_t *>(base + up(bd) + 2 * up(be));
-    uint32_t *d_off = reinterpret_cast<uint32_t *>(base + up(bd) + 3 * up(be));
-    uint32_t *d_lm = reinterpret_cast<uint32_t *>(base + up(bd) + 3 * up(be) + up(bo));
-    // Small tables go through a pinned host block (copied with the call, so the
-    // caller's arrays are free on return and the copy is truly asynchronous);
-    // when they and the buffer layout equal the previous call's (the same
-    // matrices and labels loaded again), the device copies are still there.
-    std::vector<unsigned char> key(6 * sizeof(size_t) + bd + bo + (size_t)nlm * 4);
-    {
-        const size_t head[6] = {bd, be, bo, bl, (size_t)nlm, (size_t)(uintptr_t)ctx->edge_buf.p};
-        unsigned char *k = key.data();
-        memcpy(k, head, sizeof(head));
-        memcpy(k + sizeof(head), descs.data(), bd);
-        memcpy(k + sizeof(head) + bd, label_offsets, bo);
-        if (nlm) memcpy(k + sizeof(head) + bd + bo, label_mats, (size_t)nlm * 4);
-    }
-    const bool tables_loaded = key == ctx->edge_tables_key;
-    const size_t small = up(bd) + up(bo) + up(bl);
-    if (!tables_loaded && ctx->h_small_cap < small) {
-        if (ctx->h_small) cudaFreeHost(ctx->h_small);
-        ctx->h_small = nullptr;
-        ctx->h_small_cap = 0;
-        CUDA_TRY(cudaMallocHost(&ctx->h_small, small));
-        ctx->h_small_cap = small;
-    }
-    if (!tables_loaded) {
-        ctx->edge_tables_key.clear();
-        CUDA_TRY(cudaStreamSynchronize(ctx->stream));  // previous user of h_small done
-        char *hs = reinterpret_cast<char *>(ctx->h_small);
-        memcpy(hs, descs.data(), bd);
-        memcpy(hs + up(bd), label_offsets, bo);
-        if (nlm) memcpy(hs + up(bd) + up(bo), label_mats, (size_t)nlm * 4);
-        CUDA_TRY(cudaMemcpyAsync(d_desc, hs, bd, cudaMemcpyHostToDevice, ctx->stream));
-        CUDA_TRY(cudaMemcpyAsync(d_off, hs + up(bd), bo, cudaMemcpyHostToDevice, ctx->stream));
-        if (nlm)
-            CUDA_TRY(cudaMemcpyAsync(d_lm, hs + up(bd) + up(bo), (size_t)nlm * 4, cudaMemcpyHostToDevice, ctx->stream));
-        // host-edge loads overwrite the edge arrays only, never the tables
-        ctx->edge_tables_key = std::move(key);
-    }
+    const size_t small_words = (bd + bo + (size_t)nlm * 4) / 4;
     const uint32_t *m_from = nullptr, *m_label = nullptr, *m_to = nullptr;
-    if (!on_device && read_pinned_in_place && (m_from = mapped_host_array(from, nedges)) &&
-        (m_label = mapped_host_array(label, nedges)) && (m_to = mapped_host_array(to, nedges))) {
+    const bool in_place = !on_device && read_pinned_in_place && (m_from = mapped_host_array(from, nedges)) &&
+                          (m_label = mapped_host_array(label, nedges)) && (m_to = mapped_host_array(to, nedges));
+    const bool staged = !on_device && read_pinned_in_place && !in_place && 3 * be <= kEdgeStageBytes &&
+                        ensure_edge_stage(ctx);
+    auto up = [](size_t x) { return (x + 255) & ~(size_t)255; };
+    DevMat *d_desc = nullptr;
+    uint32_t *d_from = nullptr, *d_label = nullptr, *d_to = nullptr, *d_off = nullptr, *d_lm = nullptr;
+    const bool by_param = small_words <= kSmallTable;
+    if (!by_param || !(on_device || in_place || staged)) {
+        // one device block: descs | from | label | to | offsets | label_mats
+        TRY(ctx->edge_buf.ensure(up(bd) + 3 * up(be) + up(bo) + up(bl)));
+        char *base = ctx->edge_buf.as<char>();
+        d_desc = reinterpret_cast<DevMat *>(base);
+        d_from = reinterpret_cast<uint32_t *>(base + up(bd));
+        d_label = reinterpret_cast<uint32_t *>(base + up(bd) + up(be));
+        d_to = reinterpret_cast<uint32_t *>(base + up(bd) + 2 * up(be));
+        d_off = reinterpret_cast<uint32_t *>(base + up(bd) + 3 * up(be));
+        d_lm = reinterpret_cast<uint32_t *>(base + up(bd) + 3 * up(be) + up(bo));
+    }
+    if (by_param) {
+        // (edges copied below may land where an earlier call's tables were)
+        if (d_desc) ctx->edge_tables_key.clear();
+        // the tables travel in the scatter's arguments
+        ctx->edge_tab.resize(small_words);
+        unsigned char *t = reinterpret_cast<unsigned char *>(ctx->edge_tab.data());
+        memcpy(t, descs.data(), bd);
+        memcpy(t + bd, label_offsets, bo);
+        if (nlm) memcpy(t + bd + bo, label_mats, (size_t)nlm * 4);
+        in->h_edge_tab = ctx->edge_tab.data();
+        in->edge_tab_words = (uint32_t)small_words;
+    } else {
+        // Large tables go through a pinned host block (copied with the call, so the
+        // caller's arrays are free on return and the copy is truly asynchronous);
+        // when they and the buffer layout equal the previous call's (the same
+        // matrices and labels loaded again), the device copies are still there.
+        std::vector<unsigned char> key(6 * sizeof(size_t) + bd + bo + (size_t)nlm * 4);
+        {
+            const size_t head[6] = {bd, be, bo, bl, (size_t)nlm, (size_t)(uintptr_t)ctx->edge_buf.p};
+            unsigned char *k = key.data();
+            memcpy(k, head, sizeof(head));
+            memcpy(k + sizeof(head), descs.data(), bd);
+            memcpy(k + sizeof(head) + bd, label_offsets, bo);
+            if (nlm) memcpy(k + sizeof(head) + bd + bo, label_mats, (size_t)nlm * 4);
+        }
+        const bool tables_loaded = key == ctx->edge_tables_key;
+        const size_t small = up(bd) + up(bo) + up(bl);
+        if (!tables_loaded && ctx->h_small_cap < small) {
+            if (ctx->h_small) cudaFreeHost(ctx->h_small);
+            ctx->h_small = nullptr;
+            ctx->h_small_cap = 0;
+            CUDA_TRY(cudaMallocHost(&ctx->h_small, small));
+            ctx->h_small_cap = small;
+        }
+        if (!tables_loaded) {
+            ctx->edge_tables_key.clear();
+            CUDA_TRY(cudaStreamSynchronize(ctx->stream));  // previous user of h_small done
+            char *hs = reinterpret_cast<char *>(ctx->h_small);
+            memcpy(hs, descs.data(), bd);
+            memcpy(hs + up(bd), label_offsets, bo);
+            if (nlm) memcpy(hs + up(bd) + up(bo), label_mats, (size_t)nlm * 4);
+            CUDA_TRY(cudaMemcpyAsync(d_desc, hs, bd, cudaMemcpyHostToDevice, ctx->stream));
+            CUDA_TRY(cudaMemcpyAsync(d_off, hs + up(bd), bo, cudaMemcpyHostToDevice, ctx->stream));
+            if (nlm)
+                CUDA_TRY(cudaMemcpyAsync(d_lm, hs + up(bd) + up(bo), (size_t)nlm * 4, cudaMemcpyHostToDevice,
+                                         ctx->stream));
+            // host-edge loads overwrite the edge arrays only, never the tables
+            ctx->edge_tables_key = std::move(key);
+        }
+    }
+    if (in_place) {
         d_from = const_cast<uint32_t *>(m_from);
         d_label = const_cast<uint32_t *>(m_label);
         d_to = const_cast<uint32_t *>(m_to);
+        if (read_in_place) *read_in_place = true;
+    } else if (staged) {
+        char *const h = static_cast<char *>(ctx->h_edges);
+        memcpy(h, from, be);
+        memcpy(h + be, label, be);
+        memcpy(h + 2 * be, to, be);
+        d_from = ctx->h_edges_dev;
+        d_label = d_from + nedges;
+        d_to = d_label + nedges;
         if (read_in_place) *read_in_place = true;
     } else if (on_device) {
         d_from = const_cast<uint32_t *>(from);
@@ -589,12 +644,30 @@ static int load_edges_impl(cfpq_ctx *ctx, cfpq_matrix *const *mats, size_t nmats
     TRY(use_device(ctx));
     ClosureInput in;
     memset(&in, 0, sizeof(in));
-    TRY(prepare_edges(ctx, mats, nmats, from, label, to, nedges, label_offsets, label_mats, nlabels, on_device, &in));
+    // host edges: the call synchronises, so they may be read in place, and a
+    // mapped word tells about ids out of range (the counter, kept at 0 between
+    // calls, is read only then)
+    const bool quick = !on_device && ctx->h_flag_dev;
+    TRY(prepare_edges(ctx, mats, nmats, from, label, to, nedges, label_offsets, label_mats, nlabels, on_device, &in,
+                      quick));
     if (!in.nedges) return CFPQ_OK;
-    CUDA_TRY(cudaMemsetAsync(ctx->d_bad, 0, 4, ctx->stream));
-    CUDA_TRY(launch_load_edges(in.mats, in.nmats, in.from, in.label, in.to, in.nedges, in.off, in.lm, in.nlabels,
-                               in.nlm, ctx->d_bad, ctx->stream));
-    return CFPQ_OK;
+    if (!quick) {
+        CUDA_TRY(cudaMemsetAsync(ctx->d_bad, 0, 4, ctx->stream));
+        CUDA_TRY(launch_load_edges(in, ctx->stream));
+        return on_device ? CFPQ_OK : check_bad(ctx, "cfpq_load_edges");
+    }
+    uint32_t *const h_bad = ctx->h_flag + kLoadBadSlot, *const d_count = ctx->d_bad + 1;
+    *h_bad = 0;
+    in.bad = d_count;
+    in.bad_host = ctx->h_flag_dev + kLoadBadSlot;
+    const cudaError_t e = launch_load_edges(in, ctx->stream);
+    CUDA_TRY(cudaStreamSynchronize(ctx->stream));  // also after a failed launch: the edges may be read in place
+    CUDA_TRY(e);
+    if (!*(volatile uint32_t *)h_bad) return CFPQ_OK;
+    uint32_t bad = 0;
+    CUDA_TRY(cudaMemcpy(&bad, d_count, 4, cudaMemcpyDeviceToHost));
+    CUDA_TRY(cudaMemset(d_count, 0, 4));
+    return set_error(CFPQ_ERR_INVALID, "cfpq_load_edges: %u coordinates out of range", bad);
 }
 
 extern "C" int cfpq_matrix_set_diagonal(cfpq_ctx *ctx, cfpq_matrix *m) {
@@ -611,8 +684,9 @@ extern "C" int cfpq_matrix_clear(cfpq_ctx *ctx, cfpq_matrix *m) {
     return CFPQ_OK;
 }
 
-// The clear list of `count` matrices on the device (one unit per tile-row,
-// MatRows prefix sums), re-sent only when it differs from the last one.
+// The clear list of `count` matrices (one unit per tile-row, MatRows prefix
+// sums), in the kernel's arguments or, when too long, on the device, re-sent
+// only when it differs from the last one.
 static int prepare_clear(cfpq_ctx *ctx, cfpq_matrix *const *mats, size_t count, ClosureInput *in) {
     in->clear_rows = 0;
     if (count == 0) return CFPQ_OK;
@@ -625,6 +699,13 @@ static int prepare_clear(cfpq_ctx *ctx, cfpq_matrix *const *mats, size_t count, 
         tab[i].row_start = rows;
         tab[i].pad = 0;
         rows += mats[i]->d.T;
+    }
+    in->nclear = (uint32_t)count;
+    in->clear_rows = rows;
+    if (count * (sizeof(MatRows) / 4) <= kSmallTable) {  // the list travels in the kernel's arguments
+        ctx->clear_tab = std::move(tab);
+        in->h_clear = ctx->clear_tab.data();
+        return CFPQ_OK;
     }
     void *const before = ctx->clear_desc.p;
     TRY(ctx->clear_desc.ensure(count * sizeof(MatRows)));
@@ -639,8 +720,6 @@ static int prepare_clear(cfpq_ctx *ctx, cfpq_matrix *const *mats, size_t count, 
         ctx->clear_desc_key = std::move(key);
     }
     in->clear = ctx->clear_desc.as<MatRows>();
-    in->nclear = (uint32_t)count;
-    in->clear_rows = rows;
     return CFPQ_OK;
 }
 
@@ -649,7 +728,7 @@ extern "C" int cfpq_matrices_clear(cfpq_ctx *ctx, cfpq_matrix *const *mats, size
     ClosureInput in;
     memset(&in, 0, sizeof(in));
     TRY(prepare_clear(ctx, mats, count, &in));
-    if (in.clear_rows) CUDA_TRY(launch_clear_rows(in.clear, in.nclear, in.clear_rows, ctx->stream));
+    CUDA_TRY(launch_clear_rows(in, ctx->stream));
     return CFPQ_OK;
 }
 
@@ -1237,6 +1316,7 @@ static int build_plan(cfpq_ctx *ctx, const std::vector<QueryIn> &qs, int variant
         qrange.nprod = (uint32_t)pl->prods.size() - qrange.prod0;
         pl->qranges.push_back(qrange);
     }
+    while (pl->tc_ok.size() % 4) pl->tc_ok.push_back(0);  // whole words: the table is sent by words
     pl->item_cap = std::max<size_t>(pl->item_cap, 1);
     pl->uses_tc = !pl->tc_prods.empty() && !pl->late_select;
     for (const TcProduct &tp : pl->tc_prods) {
@@ -1725,18 +1805,25 @@ static int run_engine(cfpq_ctx *ctx, const std::vector<QueryIn> &qs, const cfpq_
     qt.done_ns = ctx->qtrack.as<unsigned long long>();
     qt.changed = reinterpret_cast<uint32_t *>(qt.done_ns + nq);
     qt.last_iter = qt.changed + 3 * nq;
+    // the plan's tables: short ones in the arguments of the prologue's launch
+    // (one query's: no copies before it, 5-8 us each), else copied here
+    struct Table {
+        void *dst;
+        const void *src;
+        size_t bytes;
+    } const tables[ClosureBegin::kTables] = {{ctx->slots.p, pl.slots.data(), pl.slots.size() * sizeof(MatSlot)},
+                                             {ctx->prods.p, pl.prods.data(), pl.prods.size() * sizeof(ProdDesc)},
+                                             {ctx->tc_ok.p, pl.tc_ok.data(), pl.tc_ok.size()},
+                                             {ctx->qranges.p, pl.qranges.data(), pl.qranges.size() * sizeof(QueryRange)},
+                                             {ctx->tc_rows.p, pl.tc_rows.data(), pl.tc_rows.size() * sizeof(TcRows)}};
+    size_t table_words = 0;
+    for (const Table &t : tables) table_words += (t.bytes + 3) / 4;
+    const bool tables_by_param = !tables_current && table_words <= kLargeTable;
     if (!tables_current) {
-        CUDA_TRY(cudaMemcpyAsync(ctx->slots.p, pl.slots.data(), pl.slots.size() * sizeof(MatSlot),
-                                 cudaMemcpyHostToDevice, ctx->stream));
-        CUDA_TRY(cudaMemcpyAsync(ctx->prods.p, pl.prods.data(), pl.prods.size() * sizeof(ProdDesc),
-                                 cudaMemcpyHostToDevice, ctx->stream));
-        CUDA_TRY(cudaMemcpyAsync(ctx->tc_ok.p, pl.tc_ok.data(), nprods, cudaMemcpyHostToDevice, ctx->stream));
-        CUDA_TRY(cudaMemcpyAsync(ctx->qranges.p, pl.qranges.data(), pl.qranges.size() * sizeof(QueryRange),
-                                 cudaMemcpyHostToDevice, ctx->stream));
-        if (!pl.tc_rows.empty())
-            CUDA_TRY(cudaMemcpyAsync(ctx->tc_rows.p, pl.tc_rows.data(), pl.tc_rows.size() * sizeof(TcRows),
-                                     cudaMemcpyHostToDevice, ctx->stream));
-        ctx->tables_owner = pc.id;
+        ctx->tables_owner = 0;
+        for (const Table &t : tables)
+            if (!tables_by_param && t.bytes)
+                CUDA_TRY(cudaMemcpyAsync(t.dst, t.src, t.bytes, cudaMemcpyHostToDevice, ctx->stream));
     }
     // the persistent kernel hands its final state (and the caller's flag
     // word, which lives in the pinned flag block) to the host itself
@@ -1759,6 +1846,11 @@ static int run_engine(cfpq_ctx *ctx, const std::vector<QueryIn> &qs, const cfpq_
     b.nchoice = nprods;
     b.choice_value = pl.auto_select ? (uint8_t)CFPQ_VARIANT_LOP3 : pl.fixed_variant;
     b.st = ctx->d_st;
+    for (int k = 0; tables_by_param && k < ClosureBegin::kTables; ++k) {
+        b.table[k] = static_cast<uint32_t *>(tables[k].dst);
+        b.h_table[k] = tables[k].src;
+        b.table_words[k] = (uint32_t)((tables[k].bytes + 3) / 4);
+    }
     b.max_iter = o.max_iterations > 0 ? (uint32_t)o.max_iterations : 0;
     b.nqueries = (uint32_t)nq;
     // the query's input phase, enqueued right before the closure's own
@@ -1767,11 +1859,13 @@ static int run_engine(cfpq_ctx *ctx, const std::vector<QueryIn> &qs, const cfpq_
     // first kernel clears the matrices and runs the closure prologue, which
     // touches neither the matrices nor the counters
     if (input) CUDA_TRY(launch_closure_input(*input, ctx->num_sms, ctx->stream, &b));
+    else CUDA_TRY(launch_closure_begin(b, ctx->num_sms, ctx->stream));
+    ctx->tables_owner = pc.id;
     if (ctx->cnts_on) CUDA_TRY(launch_counters_init(ctx->slots.as<MatSlot>(), nslots, ctx->cnts.as<BufCounters>(),
                                                     false, ctx->stream));
     if (ctx->sel_log_iters)
         CUDA_TRY(cudaMemsetAsync(ctx->sel_log.p, 0, (size_t)kSelLogIters * nprods * sizeof(SelLogRow), ctx->stream));
-    if (!input) CUDA_TRY(launch_closure_begin(b, ctx->num_sms, ctx->stream));
+
     cudaGraphExec_t exec = nullptr;
     if (o.use_graph && !timed && !log_products && !persistent) TRY(get_loop_graph(ctx, pl, qt, &exec));
     if (timed) memset(&ctx->prof, 0, sizeof(ctx->prof));

@@ -147,7 +147,11 @@ struct cfpq_ctx {
     cfpq_kernel_profile prof = {};
     void *h_small = nullptr;
     size_t h_small_cap = 0;
-    std::vector<unsigned char> edge_tables_key;  // small tables of the last edge load still in edge_buf
+    std::vector<uint32_t> edge_tab;    // tables of the edge load in flight, sent in its launch
+    std::vector<MatRows> clear_tab;    // matrix list of the clear in flight, sent in its launch
+    void *h_edges = nullptr;           // pinned block of short pageable edge lists (kEdgeStageBytes)
+    uint32_t *h_edges_dev = nullptr;   // the same as the device sees it
+    std::vector<unsigned char> edge_tables_key;  // large tables of the last edge load still in edge_buf
     std::vector<unsigned char> clear_desc_key;   // matrix list of the last cfpq_matrices_clear in clear_desc
     std::vector<unsigned char> diag_desc_key;    // epsilon matrices of the last cfpq_intersection in diag_desc
     void *items_clean_ptr = nullptr;  // items buffer whose first items_clean_words words are zero

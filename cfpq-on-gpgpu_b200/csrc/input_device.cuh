@@ -23,8 +23,24 @@ struct ClosureInput {
     uint32_t nlm;
     uint32_t ndiag;
     const DevMat *diag;
-    uint32_t *bad;  // out-of-range vertex ids are counted here (and skipped)
+    uint32_t *bad;       // out-of-range vertex ids are counted here (and skipped)
+    uint32_t *bad_host;  // non-null: mapped host word set to 1 if there was one
+    // Tables that fit a kernel's arguments travel with the launch instead of
+    // being copied to the device first (host pointers; the device pointers
+    // above are then null): the clear list, and matrices, label offsets and label
+    // lists of the edge scatter laid end to end (edge_tab_words words).
+    const MatRows *h_clear;
+    const uint32_t *h_edge_tab;
+    uint32_t edge_tab_words;
 };
+
+// Table passed by value in a kernel's arguments.
+template <uint32_t kWords>
+struct alignas(16) ParamTable {
+    static constexpr uint32_t kCap = kWords;
+    uint32_t w[kWords];
+};
+constexpr uint32_t kSmallTable = 512, kLargeTable = 3072;  // words
 
 #ifdef __CUDACC__
 
@@ -53,12 +69,14 @@ __device__ __forceinline__ void set_one_bit(const DevMat &m, uint32_t r, uint32_
 // One edge (label l, r -> c) into every matrix of its label; ids out of a
 // matrix's range are counted in *bad and skipped.
 __device__ __forceinline__ void scatter_edge(const DevMat *mats, const uint32_t *off, const uint32_t *lm,
-                                             uint32_t nlabels, uint32_t l, uint32_t r, uint32_t c, uint32_t *bad) {
+                                             uint32_t nlabels, uint32_t l, uint32_t r, uint32_t c, uint32_t *bad,
+                                             uint32_t *bad_host) {
     if (l >= nlabels) return;
     for (uint32_t j = off[l]; j < off[l + 1]; ++j) {
         const DevMat m = mats[lm[j]];
         if (r >= m.n || c >= m.n) {
             atomicAdd(bad, 1u);
+            if (bad_host) *bad_host = 1u;
             continue;
         }
         set_one_bit(m, r, c);

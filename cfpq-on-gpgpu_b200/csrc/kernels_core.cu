@@ -2,6 +2,7 @@
 // bit scatter, result hash, the plain dense product, and the plan / advance
 // steps of the device-resident closure iteration.
 #include <algorithm>
+#include <cstring>
 
 #include "input_device.cuh"
 #include "launch.h"
@@ -58,20 +59,32 @@ __global__ void k_set_bits(DevMat m, const uint32_t *__restrict__ rows, const ui
 // block starts while that kernel still clears the matrices: the edge and
 // table loads, which do not depend on it, go first, and pdl_wait() keeps
 // every write to the matrices and the counter after its end.
+// Where the tables come from: kTabGlobal read in place, kTabStaged copied from
+// device memory, kTabParam copied from the kernel's arguments (small tables of a
+// query: no copy to the device before the launch, 5-8 us of stream time and
+// host time each).
 constexpr uint32_t kLoadTableBytes = 12288;
+enum : int { kTabGlobal = 0, kTabStaged = 1, kTabParam = 2 };
 
-template <bool kSmem>
-__global__ void k_load_edges(const DevMat *__restrict__ mats, uint32_t nmats, const uint32_t *__restrict__ from,
+template <int kTab>
+__global__ void k_load_edges(const __grid_constant__ ParamTable<kTab == kTabParam ? kSmallTable : 4> param,
+                             const DevMat *__restrict__ mats, uint32_t nmats, const uint32_t *__restrict__ from,
                              const uint32_t *__restrict__ label, const uint32_t *__restrict__ to, size_t ne,
                              const uint32_t *__restrict__ off, const uint32_t *__restrict__ lm, uint32_t nlabels,
-                             uint32_t nlm, uint32_t *bad) {
+                             uint32_t nlm, uint32_t *bad, uint32_t *bad_host) {
     extern __shared__ __align__(16) unsigned char load_smem[];
-    if constexpr (kSmem) {
+    if constexpr (kTab != kTabGlobal) {
         DevMat *sm = reinterpret_cast<DevMat *>(load_smem);
         uint32_t *so = reinterpret_cast<uint32_t *>(sm + nmats), *sl = so + nlabels + 1;
-        for (uint32_t i = threadIdx.x; i < nmats; i += blockDim.x) sm[i] = mats[i];
-        for (uint32_t i = threadIdx.x; i <= nlabels; i += blockDim.x) so[i] = off[i];
-        for (uint32_t i = threadIdx.x; i < nlm; i += blockDim.x) sl[i] = lm[i];
+        if constexpr (kTab == kTabParam) {
+            const uint32_t words = nmats * (uint32_t)(sizeof(DevMat) / 4) + nlabels + 1 + nlm;
+            uint32_t *dst = reinterpret_cast<uint32_t *>(load_smem);
+            for (uint32_t i = threadIdx.x; i < words; i += blockDim.x) dst[i] = param.w[i];
+        } else {
+            for (uint32_t i = threadIdx.x; i < nmats; i += blockDim.x) sm[i] = mats[i];
+            for (uint32_t i = threadIdx.x; i <= nlabels; i += blockDim.x) so[i] = off[i];
+            for (uint32_t i = threadIdx.x; i < nlm; i += blockDim.x) sl[i] = lm[i];
+        }
         mats = sm;
         off = so;
         lm = sl;
@@ -83,10 +96,10 @@ __global__ void k_load_edges(const DevMat *__restrict__ mats, uint32_t nmats, co
         r = from[e];
         c = to[e];
     }
-    if constexpr (kSmem) __syncthreads();
+    if constexpr (kTab != kTabGlobal) __syncthreads();
     pdl_wait();
     for (; e < ne; e += (size_t)gridDim.x * blockDim.x) {
-        scatter_edge(mats, off, lm, nlabels, l, r, c, bad);
+        scatter_edge(mats, off, lm, nlabels, l, r, c, bad, bad_host);
         const size_t e2 = e + (size_t)gridDim.x * blockDim.x;
         if (e2 < ne) {
             l = label[e2];
@@ -520,14 +533,20 @@ __global__ void k_advance_end(const MatSlot *__restrict__ slots, uint32_t nslots
 }
 
 // Closure prologue in one launch: zero the given word ranges, fill the
-// variant choices, initialise the iteration state and stamp its start.
-// The closure prologue's work, spread over the whole grid (block 0 also
-// initialises the iteration state; every thread of block 0 must call it).
-__device__ __forceinline__ void closure_begin_body(const ClosureBegin &a) {
+// variant choices, copy the closure's tables out of the kernel's arguments,
+// initialise the iteration state and stamp its start.  The work is spread over
+// the whole grid (block 0 also initialises the iteration state; every thread
+// of block 0 must call it).
+__device__ __forceinline__ void closure_begin_body(const ClosureBegin &a, const uint32_t *tables) {
     const size_t tid = (size_t)blockIdx.x * blockDim.x + threadIdx.x, nt = (size_t)gridDim.x * blockDim.x;
     for (int r = 0; r < ClosureBegin::kRanges; ++r)
         for (size_t i = tid; i < a.nwords[r]; i += nt) a.zero[r][i] = 0u;
     for (size_t i = tid; i < a.nchoice; i += nt) a.choice[i] = a.choice_value;
+    uint32_t at = a.table_at;
+    for (int r = 0; r < ClosureBegin::kTables; ++r) {
+        for (size_t i = tid; i < a.table_words[r]; i += nt) a.table[r][i] = tables[at + i];
+        at += a.table_words[r];
+    }
     if (blockIdx.x == 0) {
         uint32_t *w = reinterpret_cast<uint32_t *>(a.st);
         for (size_t i = threadIdx.x; i < sizeof(IterState) / 4; i += blockDim.x) w[i] = 0u;
@@ -541,24 +560,32 @@ __device__ __forceinline__ void closure_begin_body(const ClosureBegin &a) {
     }
 }
 
-__global__ void k_closure_begin(ClosureBegin a) { closure_begin_body(a); }
+template <uint32_t kWords>
+__global__ void k_closure_begin(const __grid_constant__ ParamTable<kWords> param, ClosureBegin a) {
+    closure_begin_body(a, param.w);
+}
 
-// Clear a list of matrices: one warp per (matrix, tile-row), occupied tiles only.
-__global__ void k_clear_rows(const MatRows *__restrict__ tab, uint32_t nmats, uint32_t total_rows) {
+// Clear a list of matrices: one warp per (matrix, tile-row), occupied tiles
+// only; the list in device memory (tab) or in the arguments.
+template <uint32_t kWords>
+__global__ void k_clear_rows(const __grid_constant__ ParamTable<kWords> param, const MatRows *__restrict__ tab,
+                             uint32_t nmats, uint32_t total_rows) {
     const uint32_t gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    if (gw < total_rows) clear_unit(tab, nmats, gw);
+    if (gw < total_rows) clear_unit(tab ? tab : reinterpret_cast<const MatRows *>(param.w), nmats, gw);
 }
 
 // First kernel of a query's input phase: the clear of its matrices, the
 // scatter's out-of-range counter set to 0 and (with_begin) the closure
-// prologue, in one launch ahead of the scatter.
-__global__ void k_input_first(const MatRows *__restrict__ tab, uint32_t nmats, uint32_t total_rows, uint32_t *bad,
-                              ClosureBegin begin, int with_begin) {
+// prologue, in one launch ahead of the scatter.  Arguments: the clear list
+// (unless tab is given), then the closure's tables.
+template <uint32_t kWords>
+__global__ void k_input_first(const __grid_constant__ ParamTable<kWords> param, const MatRows *__restrict__ tab,
+                              uint32_t nmats, uint32_t total_rows, uint32_t *bad, ClosureBegin begin, int with_begin) {
     pdl_launch_dependents();  // the scatter may start its loads now
     const uint32_t gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    if (gw < total_rows) clear_unit(tab, nmats, gw);
+    if (gw < total_rows) clear_unit(tab ? tab : reinterpret_cast<const MatRows *>(param.w), nmats, gw);
     if (bad && blockIdx.x == 0 && threadIdx.x == 0) *bad = 0u;
-    if (with_begin) closure_begin_body(begin);
+    if (with_begin) closure_begin_body(begin, param.w);
 }
 
 // Diagonals of a list of matrices (epsilon nonterminals).
@@ -581,14 +608,12 @@ cudaError_t launch_set_bits(const DevMat &m, const uint32_t *d_rows, const uint3
     return cudaGetLastError();
 }
 
-cudaError_t launch_load_edges(const DevMat *d_mats, uint32_t nmats, const uint32_t *d_from, const uint32_t *d_label,
-                              const uint32_t *d_to, size_t ne, const uint32_t *d_off, const uint32_t *d_lm,
-                              uint32_t nlabels, uint32_t nlm, uint32_t *d_bad, cudaStream_t s, bool dependent) {
-    if (ne == 0) return cudaSuccess;
-    const size_t tb = (size_t)nmats * sizeof(DevMat) + ((size_t)nlabels + 1 + nlm) * 4;
+cudaError_t launch_load_edges(const ClosureInput &in, cudaStream_t s, bool dependent) {
+    if (in.nedges == 0) return cudaSuccess;
+    const size_t tb = (size_t)in.nmats * sizeof(DevMat) + ((size_t)in.nlabels + 1 + in.nlm) * 4;
     const bool smem = tb <= kLoadTableBytes;
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(capped_grid(ne, 256, 65535u * 16));
+    cfg.gridDim = dim3(capped_grid(in.nedges, 256, 65535u * 16));
     cfg.blockDim = dim3(256);
     cfg.dynamicSmemBytes = smem ? tb : 0;
     cfg.stream = s;
@@ -597,10 +622,18 @@ cudaError_t launch_load_edges(const DevMat *d_mats, uint32_t nmats, const uint32
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = dependent ? 1 : 0;
-    return smem ? cudaLaunchKernelEx(&cfg, k_load_edges<true>, d_mats, nmats, d_from, d_label, d_to, ne, d_off, d_lm,
-                                     nlabels, nlm, d_bad)
-                : cudaLaunchKernelEx(&cfg, k_load_edges<false>, d_mats, nmats, d_from, d_label, d_to, ne, d_off,
-                                     d_lm, nlabels, nlm, d_bad);
+    auto launch = [&](auto kernel, const auto &param) {
+        return cudaLaunchKernelEx(&cfg, kernel, param, in.mats, in.nmats, in.from, in.label, in.to, in.nedges, in.off,
+                                  in.lm, in.nlabels, in.nlm, in.bad, in.bad_host);
+    };
+    if (in.h_edge_tab) {
+        if (in.edge_tab_words > kSmallTable || !smem) return cudaErrorInvalidValue;
+        ParamTable<kSmallTable> p;
+        memcpy(p.w, in.h_edge_tab, (size_t)in.edge_tab_words * 4);
+        return launch(k_load_edges<kTabParam>, p);
+    }
+    const ParamTable<4> none{};
+    return smem ? launch(k_load_edges<kTabStaged>, none) : launch(k_load_edges<kTabGlobal>, none);
 }
 
 cudaError_t launch_set_diag(const DevMat &m, cudaStream_t s) {
@@ -781,33 +814,76 @@ cudaError_t launch_advance_end(const MatSlot *d_slots, uint32_t nslots, uint32_t
     return cudaGetLastError();
 }
 
-cudaError_t launch_clear_rows(const MatRows *d_tab, uint32_t nmats, uint32_t total_rows, cudaStream_t s) {
-    if (total_rows == 0 || nmats == 0) return cudaSuccess;
-    k_clear_rows<<<grid_for((size_t)total_rows * 32, 256), 256, 0, s>>>(d_tab, nmats, total_rows);
+cudaError_t launch_clear_rows(const ClosureInput &in, cudaStream_t s) {
+    if (in.clear_rows == 0 || in.nclear == 0) return cudaSuccess;
+    const unsigned grid = grid_for((size_t)in.clear_rows * 32, 256);
+    const size_t words = (size_t)in.nclear * (sizeof(MatRows) / 4);
+    if (!in.h_clear) {
+        k_clear_rows<4><<<grid, 256, 0, s>>>(ParamTable<4>{}, in.clear, in.nclear, in.clear_rows);
+    } else if (words <= kSmallTable) {
+        ParamTable<kSmallTable> p;
+        memcpy(p.w, in.h_clear, words * 4);
+        k_clear_rows<kSmallTable><<<grid, 256, 0, s>>>(p, nullptr, in.nclear, in.clear_rows);
+    } else {
+        return cudaErrorInvalidValue;
+    }
     return cudaGetLastError();
 }
 
 static unsigned closure_begin_blocks(const ClosureBegin &a, int num_sms) {
     size_t words = a.nchoice;
     for (int r = 0; r < ClosureBegin::kRanges; ++r) words = words > a.nwords[r] ? words : a.nwords[r];
+    for (int r = 0; r < ClosureBegin::kTables; ++r) words = words > a.table_words[r] ? words : a.table_words[r];
     return (unsigned)std::max<size_t>(1, std::min<size_t>((words + 255) / 256, (size_t)num_sms * 4));
 }
 
+static size_t begin_table_words(const ClosureBegin *b) {
+    size_t words = 0;
+    for (int r = 0; b && r < ClosureBegin::kTables; ++r) words += b->table_words[r];
+    return words;
+}
+
+// The closure's tables behind the first `at` words of p.
+static void append_tables(uint32_t *p, size_t at, const ClosureBegin &b) {
+    for (int r = 0; r < ClosureBegin::kTables; ++r) {
+        if (b.table_words[r]) memcpy(p + at, b.h_table[r], (size_t)b.table_words[r] * 4);
+        at += b.table_words[r];
+    }
+}
+
+template <uint32_t kWords>
+static void launch_input_first(const ClosureInput &in, unsigned blocks, const ClosureBegin *begin, size_t clear_words,
+                               cudaStream_t s) {
+    ParamTable<kWords> p;
+    if (clear_words) memcpy(p.w, in.h_clear, clear_words * 4);
+    ClosureBegin b;
+    memset(&b, 0, sizeof(b));
+    if (begin) {
+        b = *begin;
+        b.table_at = (uint32_t)clear_words;
+        append_tables(p.w, clear_words, b);
+    }
+    k_input_first<kWords><<<blocks, 256, 0, s>>>(p, in.h_clear ? nullptr : in.clear, in.nclear,
+                                                 in.nclear ? in.clear_rows : 0, in.bad, b, begin ? 1 : 0);
+}
+
 cudaError_t launch_closure_input(const ClosureInput &in, int num_sms, cudaStream_t s, const ClosureBegin *begin) {
-    if (in.clear_rows || in.bad || begin) {
+    const bool first_launched = in.clear_rows || in.bad || begin;
+    if (first_launched) {
         const unsigned clear_blocks = in.clear_rows && in.nclear ? grid_for((size_t)in.clear_rows * 32, 256) : 1;
         const unsigned blocks = begin ? std::max(clear_blocks, closure_begin_blocks(*begin, num_sms)) : clear_blocks;
-        ClosureBegin none;
-        memset(&none, 0, sizeof(none));
-        k_input_first<<<blocks, 256, 0, s>>>(in.clear, in.nclear, in.nclear ? in.clear_rows : 0, in.bad,
-                                             begin ? *begin : none, begin ? 1 : 0);
+        const size_t clear_words = in.h_clear ? (size_t)in.nclear * (sizeof(MatRows) / 4) : 0;
+        const size_t words = clear_words + begin_table_words(begin);
+        if (words <= 4) launch_input_first<4>(in, blocks, begin, clear_words, s);
+        else if (words <= kSmallTable) launch_input_first<kSmallTable>(in, blocks, begin, clear_words, s);
+        else if (words <= kSmallTable + kLargeTable)
+            launch_input_first<kSmallTable + kLargeTable>(in, blocks, begin, clear_words, s);
+        else return cudaErrorInvalidValue;
         cudaError_t e = cudaGetLastError();
         if (e != cudaSuccess) return e;
     }
-    const bool first_launched = in.clear_rows || in.bad || begin;
     if (in.nedges) {
-        cudaError_t e = launch_load_edges(in.mats, in.nmats, in.from, in.label, in.to, in.nedges, in.off, in.lm,
-                                          in.nlabels, in.nlm, in.bad, s, first_launched);
+        cudaError_t e = launch_load_edges(in, s, first_launched);
         if (e != cudaSuccess) return e;
     }
     if (in.ndiag) {
@@ -817,8 +893,22 @@ cudaError_t launch_closure_input(const ClosureInput &in, int num_sms, cudaStream
     return cudaSuccess;
 }
 
+template <uint32_t kWords>
+static void launch_begin(const ClosureBegin &a, unsigned blocks, cudaStream_t s) {
+    ParamTable<kWords> p;
+    ClosureBegin b = a;
+    b.table_at = 0;
+    append_tables(p.w, 0, b);
+    k_closure_begin<kWords><<<blocks, 256, 0, s>>>(p, b);
+}
+
 cudaError_t launch_closure_begin(const ClosureBegin &a, int num_sms, cudaStream_t s) {
-    k_closure_begin<<<closure_begin_blocks(a, num_sms), 256, 0, s>>>(a);
+    const unsigned blocks = closure_begin_blocks(a, num_sms);
+    const size_t words = begin_table_words(&a);
+    if (words <= 4) launch_begin<4>(a, blocks, s);
+    else if (words <= kSmallTable) launch_begin<kSmallTable>(a, blocks, s);
+    else if (words <= kLargeTable) launch_begin<kLargeTable>(a, blocks, s);
+    else return cudaErrorInvalidValue;
     return cudaGetLastError();
 }
 

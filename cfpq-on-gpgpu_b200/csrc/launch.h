@@ -12,11 +12,10 @@ namespace cfpq {
 // Layout / initialisation
 cudaError_t launch_set_bits(const DevMat &m, const uint32_t *d_rows, const uint32_t *d_cols, size_t count,
                             uint32_t *d_bad, cudaStream_t s);
-// dependent: launched right after k_input_first as a programmatic dependent
-// launch (its loads of edges and tables overlap that kernel).
-cudaError_t launch_load_edges(const DevMat *d_mats, uint32_t nmats, const uint32_t *d_from, const uint32_t *d_label,
-                              const uint32_t *d_to, size_t ne, const uint32_t *d_off, const uint32_t *d_lm,
-                              uint32_t nlabels, uint32_t nlm, uint32_t *d_bad, cudaStream_t s, bool dependent = false);
+// Edge scatter of `in` (its edge fields).  dependent: launched right after
+// k_input_first as a programmatic dependent launch (its loads of edges and
+// tables overlap that kernel).
+cudaError_t launch_load_edges(const ClosureInput &in, cudaStream_t s, bool dependent = false);
 cudaError_t launch_set_diag(const DevMat &m, cudaStream_t s);
 cudaError_t launch_occ_rebuild(const DevMat &m, cudaStream_t s);
 // delta = cur & ~prev, then prev = cur; tile statistics of both rebuilt.
@@ -41,8 +40,10 @@ cudaError_t launch_copy_matrix(const DevMat &dst, const DevMat &src, cudaStream_
 cudaError_t launch_clear_matrix(const DevMat &m, cudaStream_t s);
 // Seeded random matrix with the given bit density (not for ordered matrices).
 cudaError_t launch_random_fill(const DevMat &m, double density, uint64_t seed, cudaStream_t s);
-// Clear the matrices of d_tab (occupied tiles only; relies on the occupancy invariant).
-cudaError_t launch_clear_rows(const MatRows *d_tab, uint32_t nmats, uint32_t total_rows, cudaStream_t s);
+// Clear the matrices of in's clear list (occupied tiles only; relies on the
+// occupancy invariant).  A list in the arguments (in.h_clear) has at most
+// kSmallTable words.
+cudaError_t launch_clear_rows(const ClosureInput &in, cudaStream_t s);
 
 // Result hash / count (cfpq-cpp/Grammar.cpp:81-100 on the device) of up to
 // kHashBatch matrices in one launch: one block per tile-row (matrix i owns
@@ -133,8 +134,8 @@ cudaError_t launch_advance_end(const MatSlot *d_slots, uint32_t nslots, uint32_t
                                BufCounters *d_cnts, cudaStream_t s);
 
 // Closure prologue (one launch): zero[r][0 .. nwords[r]) = 0, choice[0 ..
-// nchoice) = choice_value, *st = a fresh iteration state (active, max_iter,
-// nqueries, start stamp).
+// nchoice) = choice_value, table[r] = h_table[r], *st = a fresh iteration state
+// (active, max_iter, nqueries, start stamp).
 struct ClosureBegin {
     static constexpr int kRanges = 3;
     uint32_t *zero[kRanges];
@@ -144,6 +145,13 @@ struct ClosureBegin {
     uint8_t choice_value;
     IterState *st;
     uint32_t max_iter, nqueries;
+    // host tables copied to table[r] from the kernel's arguments (kLargeTable
+    // words at most), where they start at word table_at
+    static constexpr int kTables = 5;
+    uint32_t *table[kTables];
+    const void *h_table[kTables];
+    uint32_t table_words[kTables];
+    uint32_t table_at;
 };
 cudaError_t launch_closure_begin(const ClosureBegin &a, int num_sms, cudaStream_t s);
 // A query's input phase as stand-alone kernels: clear (with in.bad set to 0
