@@ -1,44 +1,62 @@
 // Variant TC: exact Boolean product C |= P * Q on the 5th-generation tensor
-// cores (tcgen05.mma kind::i8, 0/1 operands, int32 accumulators in TMEM,
-// result bit = accumulator > 0).
+// cores (tcgen05.mma kind::mxf4: 4-bit operands that are non-zero where the bit
+// is set, all scales 1, fp32 accumulators in TMEM, result bit = accumulator !=
+// 0).  Every product is 0 or in [1/4, 4] and a sum has at most 2^17 of them, all
+// of one sign: a sum is zero exactly where every product is, in any rounding.
 //
-// Operands travel as packed bits and are expanded on chip.  Per k-tile tk of
-// a work item the copy warp stages the 4 P tiles (ti0..ti0+3, tk) and the Q
-// block (tk, tj0..tj0+3) -- 4 KiB of bits, bulk copies completing on the
-// stage's mbarrier -- into one of kPkStages packed stages.  Sixteen expander
-// warps in two groups of eight (group g takes the k-tiles of parity g, so a
-// warp has two k-tiles' time for each of its expansions) turn a packed stage
-// into the MMA operands in one of kOpStages operand stages: warp w < 4 of a
-// group writes P tile w as 0/1 bytes by rows (64 rows x 64 k)
-// in the canonical no-swizzle K-major layout (8-row x 16-byte core matrices,
-// K-adjacent core matrices 128 B apart, 8-row groups 512 B apart), warp
-// w >= 4 writes Q tile w-4 by its rows (k) in the MN-major layout (16 output
-// columns x 8 k-rows per 128-byte core matrix, column groups 128 B apart,
-// 8-row k groups 2048 B apart), so neither operand is transposed; each
-// nibble of bits becomes 4 bytes of 0/1 by one multiply and one mask.
-// The warps then fence the writes for the async proxy and arrive on the
-// operand stage's "full" barrier.  The MMA warp issues 4
-// tcgen05.mma per k-tile (2 accumulators of M=128 x N=256, 2 K-halves of 32)
-// and commits them to the operand stage's "empty" barrier, which the
-// expanders wait on before reusing it; after the item's last k-tile a commit
-// to the accumulator barrier releases the epilogue.  Global memory only ever
-// supplies packed bits (512 B per 64x64 tile): the operands of a dense
-// n = 8192 product are 16 MiB and stay in L2.
+// Operands travel as packed bits and are expanded on chip.  A bit keeps its
+// place in a nibble: word w of the 4 words of 32 bits x is x & 0x11111111,
+// x & 0x22222222, x & 0x44444444, (x >> 3) & 0x11111111 (E2M1 codes 1, 2, 4 =
+// 1/2, 1, 2; code 8 would be -0).  The order of k inside 64 is then a permuted
+// one, the same for both operands.
 //
-// Work item (item list 2) = (product, group of 4 output tile-rows, block of 4
-// output tiles): a 256 x 256-bit output block over the whole inner dimension,
-// accumulated in TMEM as two 128 x 256 int32 matrices (all 512 TMEM columns;
-// one CTA per SM).  Epilogue (the 16 expander warps): tcgen05.ld 32x32b.x32
-// (warp w reads accumulator (w/4)%2, TMEM lanes 32*(w%4).., output tiles
-// 2*(w/8) and 2*(w/8)+1 of the block), threshold > 0, pack 64 columns into a
-// word, then the atomic-OR epilogue of the word-level kernels (C, next delta
-// D, occupancy, populations).
+// 4-bit operands are K-major on both sides, so one of them has to be transposed
+// bit by bit.  The block is computed as C^T = Q^T P^T: M is 128 columns of Q (2
+// tiles), N is 256 rows of P (4 tiles), and it is the smaller side that is
+// transposed, in registers (transpose_rows, 5 shuffles per 64 x 32 bits).  Work
+// item (item list 2) = (product, group of 4 output tile-rows, block of 4 output
+// tiles), done as two halves of 2 tile columns over the whole inner dimension.
 //
-// Arithmetic: 256*256*64 MACs per k-tile; bound = the tensor pipe's dense int8
-// rate.  Every wait is bounded; a wait that gives up raises the CTA's abort
-// flag (which ends every other role's waits), the CTA then waits (bounded) for
-// each bulk copy and MMA still in flight, frees TMEM and reports
-// CFPQ_ERR_TIMEOUT.
+// Roles (one CTA per SM, 26 warps):
+//   list warp  claims items and writes the halves' k-lists (tk with an occupied
+//              P tile and a non-empty Q half) into one of two list slots, an item
+//              ahead: it claims when the MMAs of an item's last half start;
+//   A warps    2 groups x 8: 32 columns of Q for half of a stage's k-tiles,
+//              transposed and expanded to TENSOR MEMORY (tcgen05.st), from where
+//              the MMA takes A;
+//   B warps    2 groups x 4: one tile row of P each, expanded to shared memory
+//              (no-swizzle K-major: 8-row x 16-byte core matrices);
+//              group g takes the operand stages of parity g (kKt k-tiles each),
+//              with the packed words loaded from global memory (L2) one unit of
+//              kUnit k-tiles ahead, in the registers that the last unit left;
+//   MMA warp   one tcgen05.mma (128 x 256 x 64) per k-tile, one commit per stage;
+//   epilogue   the first 16 expander warps (the A warps), each after its group's
+//              first stage of the next half, so that the stages fill while the
+//              last MMAs drain: accumulators -> bits (64 columns a warp, transposed
+//              back by shuffles) -> 4 KiB of shared memory, which frees the
+//              accumulator; then one 64-bit word a lane through the atomic-OR
+//              epilogue of the word-level kernels.
+//
+// Why this split (dense product at n = 8192, one call, 2^39 bit-MACs):
+//   525 us  kind::i8, a 256 x 256 block, both operands as bytes in shared memory,
+//           packed tiles by bulk copies: five copies per k-tile from one thread
+//           took 1088 clocks, twice the MMAs (512);
+//   408 us  128 x 256 halves with A in TMEM, words loaded straight from L2, 4
+//           k-tiles per stage: a stage's 8 MMAs cost 131 clocks each where 4 per
+//           commit cost 212 (one commit per about 600 clocks whatever the number
+//           of stages); bound by shared memory, 128 KiB a stage at 128 B/clk;
+//   262 us  4-bit operands: half the bytes through shared memory and twice the
+//           MMA rate (measured 16.1 k MAC/clk per SM against 8.0 k).
+// Now the integer ALU pipe bounds it: about 340 ALU instructions per k-tile (160
+// for the transposed side, 80 for the plain one, 40 for the epilogue) keep it
+// 70% busy and the tensor pipe 52%; the loads move 1.2 GB from L2 in that time.
+//
+// TMEM: accumulator 256 columns, kOpStages A stages of 8 columns a k-tile, 32
+// columns of scale factors.
+//
+// Every wait is bounded; a wait that gives up raises the CTA's abort flag
+// (which ends every other role's waits), the CTA then waits (bounded) for each
+// MMA still in flight, frees TMEM and reports CFPQ_ERR_TIMEOUT.
 #include <algorithm>
 
 #include "launch.h"
@@ -47,43 +65,55 @@ namespace cfpq {
 
 namespace {
 
-constexpr int kGroupWarps = 8;           // expanders of one k-tile: 4 P tiles, 4 Q tiles
-constexpr int kExpWarps = 2 * kGroupWarps;  // two groups (k-tile parity), then the epilogue
-constexpr int kCopyWarp = kExpWarps;     // lane 0 issues the bulk copies
-constexpr int kMmaWarp = kExpWarps + 1;  // lane 0 issues the MMAs
+constexpr int kAWarps = 8, kBWarps = 4;      // expanders of one stage: 128 columns of Q, 256 rows of P
+constexpr int kGroupWarps = kAWarps + kBWarps;
+constexpr int kBFirst = 2 * kAWarps;         // warps 0-7, 8-15: A of groups 0, 1; 16-19, 20-23: B
+constexpr int kExpWarps = 2 * kGroupWarps;
+constexpr int kEpiWarps = 16;                // 4 TMEM lane quarters x 4 P tiles
+constexpr int kMmaWarp = kExpWarps;          // lane 0 issues the MMAs
+constexpr int kListWarp = kExpWarps + 1;
 constexpr int kThreads = 32 * (kExpWarps + 2);
 constexpr int kMaxTiles = 2048;
-constexpr uint32_t kTmemCols = 512;
 constexpr unsigned kFull = 0xffffffffu;
-constexpr uint32_t kOperandBytes = 256 * 64;  // one operand, one stage: 256 rows x 64 bytes
-constexpr uint32_t kPkStages = 8;             // packed k-tiles in flight (4 KiB each)
-constexpr uint32_t kOpStages = 3;             // expanded operand stages (32 KiB each)
+constexpr uint32_t kN = 256;                 // output rows of an item
+constexpr uint32_t kKt = 8;                  // k-tiles per operand stage: 8 MMAs per commit
+constexpr uint32_t kUnit = 4;                // k-tiles whose packed words a lane holds ahead
+constexpr uint32_t kOpStages = 3;            // operand stages (64 KiB and 64 TMEM columns each)
+constexpr uint32_t kBTile = kN * 32;         // B operand of one k-tile
+constexpr uint32_t kTmemCols = 512;
+constexpr uint32_t kACol = kN, kACols = kKt * 8;         // A stages
+constexpr uint32_t kSfCol = kACol + kOpStages * kACols;  // scale factors of A (16 columns) and B (16)
+static_assert(kSfCol + 32 <= kTmemCols, "TMEM columns");
 
-// Instruction descriptor, kind::i8: D = S32 (bits 4-5 = 2), A = B = U8 (0),
-// A K-major (bit 15 = 0), B MN-major (bit 16 = 1), N = 256 (bits 17-22 =
-// N/8), M = 128 (bits 24-28 = M/16).
-constexpr uint32_t kIdesc = (2u << 4) | (1u << 16) | ((256u / 8) << 17) | ((128u / 16) << 24);
-// B operand (MN-major, no swizzle): 16-column groups 128 B apart (SBO),
-// 8-row k groups 2048 B apart (LBO).
-constexpr uint32_t kBSbo = 128, kBLbo = 2048;
+// Instruction descriptor, kind::mxf4: A = B = E2M1 (bits 7-9, 10-11 = 1), both
+// K-major (bits 15, 16 = 0), N (bits 17-22 = N/8), scales UE8M0 (bit 23), M =
+// 128 (bits 24-28 = M/16), K = 64 (bit 31 = 0).
+constexpr uint32_t kIdesc = (1u << 7) | (1u << 10) | ((kN / 8) << 17) | (1u << 23) | ((128u / 16) << 24);
+// B operand (K-major, no swizzle): the two 16-byte chunks of a row 128 B apart
+// (LBO), 8-row groups 256 B apart (SBO).
+constexpr uint32_t kBLbo = 128, kBSbo = 256;
+
+// One item's k-lists and matrices, written by the list warp.
+struct ListSlot {
+    alignas(8) uint16_t ktile[2][kMaxTiles];  // padded to whole units
+    uint32_t nk[2];
+    uint32_t last;  // the claims ended: no item
+    uint32_t ti0, tj0, T, head, query;
+    const uint64_t *p, *q;
+    DevMat c, d;
+};
 
 struct __align__(1024) TcSmem {
-    uint8_t a[kOpStages][kOperandBytes];  // P rows of 4 tile-rows, 4 x 4 KiB per stage
-    uint8_t b[kOpStages][kOperandBytes];  // Q^T of 4 tiles, 4 x 4 KiB per stage
-    uint64_t pk[kPkStages][8][64];        // packed: P tiles 0..3, then Q tiles 0..3
-    uint64_t pk_full[kPkStages], pk_empty[kPkStages];
+    uint8_t b[kOpStages][kKt * kBTile];  // P rows of kKt x 4 tiles
+    uint32_t out[2][4][kN];              // result bits by lane quarter and row, alternate halves
+    ListSlot list[2];
     uint64_t op_full[kOpStages], op_empty[kOpStages];
-    uint64_t acc_full;
+    uint64_t list_full[2], list_empty[2], claim;
+    uint64_t acc_full, acc_empty;
     uint32_t tmem_base;
-    uint32_t item;
-    uint32_t abort;    // a role's wait gave up: every other wait ends too
-    uint32_t pk_seen[2];  // group g: 1 + the last packed stage its warp 0 saw land (sequence number)
-    uint16_t cand[kMaxTiles];
-    uint16_t cmask[kMaxTiles];
-    uint16_t ktile[kMaxTiles];
-    uint32_t rball[kMaxTiles / 32], roff[kMaxTiles / 32];
-    uint32_t nc, nk;
+    uint32_t abort;  // a role's wait gave up: every other wait ends too
 };
+static_assert(sizeof(TcSmem) <= 227 * 1024, "shared memory");
 
 __device__ __forceinline__ DevMat resolve_operand(const MatSlot &s, uint8_t use_delta, uint32_t iter) {
     if (!use_delta || iter == 0) return s.cur;
@@ -96,11 +126,14 @@ __device__ __forceinline__ uint64_t smem_desc(uint32_t addr, uint32_t lbo, uint3
            (1ULL << 46);
 }
 
-__device__ __forceinline__ void mma_i8(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t accumulate) {
+// D (TMEM) += A (TMEM, rows = lanes, 8 k per column) * B (shared memory)
+__device__ __forceinline__ void mma_fp4(uint32_t tmem_d, uint32_t tmem_a, uint64_t bdesc, uint32_t tmem_sf,
+                                        uint32_t accumulate) {
     asm volatile(
-        "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
-        " tcgen05.mma.cta_group::1.kind::i8 [%0], %1, %2, %3, p;\n}" ::"r"(tmem_d),
-        "l"(adesc), "l"(bdesc), "r"(kIdesc), "r"(accumulate)
+        "{\n .reg .pred p;\n setp.ne.b32 p, %6, 0;\n"
+        " tcgen05.mma.cta_group::1.kind::mxf4.block_scale.scale_vec::2X [%0], [%1], %2, %3, [%4], [%5], p;\n}" ::"r"(
+            tmem_d),
+        "r"(tmem_a), "l"(bdesc), "r"(kIdesc), "r"(tmem_sf), "r"(tmem_sf + 16), "r"(accumulate)
         : "memory");
 }
 
@@ -130,34 +163,100 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&r)[32]) {
     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 }
 
-// 16 bits of `bits` starting at bit 16*c -> 16 bytes of 0/1 (bit i -> byte
-// i): each nibble times 0x00204081 puts its bits at 0, 8, 16, 24 without
-// overlapping sums; the mask keeps them.
-__device__ __forceinline__ uint4 expand16(uint64_t bits, int c) {
-    const uint32_t x = (uint32_t)(bits >> (16 * c));
-    uint4 v;
-    v.x = ((x & 15u) * 0x00204081u) & 0x01010101u;
-    v.y = (((x >> 4) & 15u) * 0x00204081u) & 0x01010101u;
-    v.z = (((x >> 8) & 15u) * 0x00204081u) & 0x01010101u;
-    v.w = (((x >> 12) & 15u) * 0x00204081u) & 0x01010101u;
-    return v;
+// 32 registers -> the lane's TMEM row, 32 columns from taddr on.
+__device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t (&r)[32]) {
+    asm volatile(
+        "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], "
+        "{%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16,"
+        "%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31,%32};" ::"r"(taddr),
+        "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]),
+        "r"(r[8]), "r"(r[9]), "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]),
+        "r"(r[16]), "r"(r[17]), "r"(r[18]), "r"(r[19]), "r"(r[20]), "r"(r[21]), "r"(r[22]), "r"(r[23]),
+        "r"(r[24]), "r"(r[25]), "r"(r[26]), "r"(r[27]), "r"(r[28]), "r"(r[29]), "r"(r[30]), "r"(r[31])
+        : "memory");
 }
 
-// A operand (K-major), operand row r (0..63) of a 4 KiB block: its 64 k-bytes
-// as 4 16-byte chunks at ((r/8)*4 + kg)*128 + (r%8)*16.
-__device__ __forceinline__ void store_row_k(uint8_t *block, uint32_t r, uint64_t bits) {
-    uint8_t *base = block + (r >> 3) * 512 + (r & 7) * 16;
-#pragma unroll
-    for (int kg = 0; kg < 4; ++kg) *reinterpret_cast<uint4 *>(base + kg * 128) = expand16(bits, kg);
+// 64 bits -> 64 nibbles (8 words), non-zero where the bit is set.
+__device__ __forceinline__ void expand64(uint32_t lo, uint32_t hi, uint32_t *r) {
+    r[0] = lo & 0x11111111u;
+    r[1] = lo & 0x22222222u;
+    r[2] = lo & 0x44444444u;
+    r[3] = (lo >> 3) & 0x11111111u;
+    r[4] = hi & 0x11111111u;
+    r[5] = hi & 0x22222222u;
+    r[6] = hi & 0x44444444u;
+    r[7] = (hi >> 3) & 0x11111111u;
 }
 
-// B operand (MN-major), k-row k (0..63) of Q tile j (output columns
-// 64j .. 64j+63): 16-column chunk c of the row at
-// (4j + c)*kBSbo + (k/8)*kBLbo + (k%8)*16.
-__device__ __forceinline__ void store_row_mn(uint8_t *b, uint32_t j, uint32_t k, uint64_t bits) {
-    uint8_t *base = b + (k >> 3) * kBLbo + (k & 7) * 16 + 4 * j * kBSbo;
+// Transpose of 64 rows x 32 columns of bits, kUnit of them side by side so that
+// the shuffles overlap: lane l holds rows first_row(l) and first_row(l) + 16 and
+// gets column l, rows 0..31 in x[.][0] and 32..63 in x[.][1].  Step i = 4..0
+// swaps the register bit of the index with bit i of the position in the word,
+// then with bit i of the lane; the row bits so move through the register into the
+// word, one place down each.  A lane with bit i set keeps the other register of
+// the two, and the registers' order is put right by the next step's selectors.
+struct Transposer {
+    uint32_t keep4, send4, keep3, send3;  // byte selectors of steps 4 and 3
+    uint32_t mask[3];                     // steps 0..2: bits of the lane's kept word that stay in place
+    uint32_t lane;
+    __device__ __forceinline__ explicit Transposer(uint32_t l) : lane(l) {
+        const bool up4 = l & 16u, up3 = l & 8u;
+        keep4 = up4 ? 0x7632u : 0x5410u;
+        send4 = up4 ? 0x5410u : 0x7632u;
+        keep3 = (up3 ? 0x7351u : 0x6240u) ^ (up4 ? 0x4444u : 0u);
+        send3 = (up3 ? 0x6240u : 0x7351u) ^ (up4 ? 0x4444u : 0u);
+        mask[2] = (l & 4u) ? 0xf0f0f0f0u : 0x0f0f0f0fu;
+        mask[1] = (l & 2u) ? 0xccccccccu : 0x33333333u;
+        mask[0] = (l & 1u) ? 0xaaaaaaaau : 0x55555555u;
+    }
+    static __device__ __forceinline__ uint32_t first_row(uint32_t l) { return (l >> 1) + (l & 1u) * 32; }
+    __device__ __forceinline__ void operator()(uint32_t (&x)[kUnit][4]) const {
 #pragma unroll
-    for (int c = 0; c < 4; ++c) *reinterpret_cast<uint4 *>(base + c * kBSbo) = expand16(bits, c);
+        for (uint32_t k = 0; k < kUnit; ++k) {
+            const uint32_t kept = __byte_perm(x[k][0], x[k][1], keep4), sent = __byte_perm(x[k][0], x[k][1], send4);
+            x[k][0] = kept;
+            x[k][1] = __shfl_xor_sync(kFull, sent, 16);
+        }
+#pragma unroll
+        for (uint32_t k = 0; k < kUnit; ++k) {
+            const uint32_t kept = __byte_perm(x[k][0], x[k][1], keep3), sent = __byte_perm(x[k][0], x[k][1], send3);
+            x[k][0] = kept;
+            x[k][1] = __shfl_xor_sync(kFull, sent, 8);
+        }
+#pragma unroll
+        for (int i = 2; i >= 0; --i) {
+            const bool swap = ((lane >> i) ^ (lane >> (i + 1))) & 1u;
+            const uint32_t s = ((lane >> i) & 1u) ? 32u - (1u << i) : 1u << i, m = mask[i];
+#pragma unroll
+            for (uint32_t k = 0; k < kUnit; ++k) {
+                const uint32_t a = swap ? x[k][1] : x[k][0], b = swap ? x[k][0] : x[k][1];
+                x[k][0] = (a & m) | (__funnelshift_l(b, b, s) & ~m);
+                x[k][1] = __shfl_xor_sync(kFull, (__funnelshift_r(a, a, s) & m) | (b & ~m), 1 << i);
+            }
+        }
+#pragma unroll
+        for (uint32_t k = 0; k < kUnit; ++k) {
+            const uint32_t a = x[k][0], b = x[k][1];
+            x[k][0] = (lane & 1u) ? b : a;
+            x[k][1] = (lane & 1u) ? a : b;
+        }
+    }
+};
+
+// Transpose of 32 x 32 bits: lane l holds row l and gets column l.
+__device__ __forceinline__ uint32_t transpose32(uint32_t x, uint32_t lane) {
+#pragma unroll
+    for (int i = 4; i >= 0; --i) {
+        const uint32_t s = 1u << i;
+        const uint32_t m = i == 4   ? 0x0000ffffu
+                           : i == 3 ? 0x00ff00ffu
+                           : i == 2 ? 0x0f0f0f0fu
+                           : i == 1 ? 0x33333333u
+                                    : 0x55555555u;
+        const uint32_t y = __shfl_xor_sync(kFull, x, s);
+        x = (lane & s) ? (x & ~m) | ((y >> s) & m) : (x & m) | ((y << s) & ~m);
+    }
+    return x;
 }
 
 // Bounded wait that also ends when another role raised the abort flag.
@@ -166,6 +265,13 @@ __device__ __forceinline__ bool wait_or_abort(uint64_t *bar, uint32_t parity, co
         if (mbar_try_wait(bar, parity)) return true;
         if ((i & 63u) == 63u && *abort) return false;
     }
+    return false;
+}
+
+// A whole warp's wait: one lane giving up ends the warp's loop and the CTA.
+__device__ __forceinline__ bool warp_wait(uint64_t *bar, uint32_t parity, volatile uint32_t *abort) {
+    if (__all_sync(kFull, wait_or_abort(bar, parity, abort))) return true;
+    *abort = 1;
     return false;
 }
 
@@ -188,7 +294,6 @@ __global__ void __launch_bounds__(kThreads, 1)
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     TcSmem &S = *reinterpret_cast<TcSmem *>(smem_raw);
     const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const uint64_t *items = items_all + 2 * list_cap;
     volatile uint32_t *abort = &S.abort;
 
     if (warp == 0) {
@@ -198,306 +303,392 @@ __global__ void __launch_bounds__(kThreads, 1)
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
     if (tid == 0) {
-        for (uint32_t s = 0; s < kPkStages; ++s) {
-            mbar_init(&S.pk_full[s], 1);
-            mbar_init(&S.pk_empty[s], kGroupWarps);
-        }
         for (uint32_t s = 0; s < kOpStages; ++s) {
             mbar_init(&S.op_full[s], kGroupWarps);
             mbar_init(&S.op_empty[s], 1);
         }
+        for (uint32_t s = 0; s < 2; ++s) {
+            mbar_init(&S.list_full[s], 1);
+            mbar_init(&S.list_empty[s], kExpWarps + 1);
+        }
+        mbar_init(&S.claim, 1);
         mbar_init(&S.acc_full, 1);
+        mbar_init(&S.acc_empty, kEpiWarps);
         S.abort = 0;
-        S.pk_seen[0] = S.pk_seen[1] = 0;
         fence_mbar_init();
     }
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = S.tmem_base;
+    if (warp < 4) {  // scale factors: 1 in every byte
+        uint32_t ones[32];
+#pragma unroll
+        for (int i = 0; i < 32; ++i) ones[i] = 0x7f7f7f7fu;
+        tmem_st32(tmem + ((32 * warp) << 16) + kSfCol, ones);
+        asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+    }
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+
     const uint32_t iter = kSingle ? 0u : st->iter;
-    const uint32_t single_blocks = (single.a.T + 3) / 4;
-    const uint32_t nitems = kSingle ? single_blocks * single_blocks : st->item_count[2];
     unsigned long long triples = 0, outw = 0, neww = 0;
-    // k-tile sequence numbers across the CTA's items: stage = seq % stages,
-    // use = seq / stages; a "full" barrier is waited with parity use & 1, an
-    // "empty" one with (use & 1) ^ 1 (a fresh barrier counts its previous
-    // phase as complete, so the first use of every stage passes)
-    uint32_t seq = 0, items_done = 0;
-    uint32_t pk_issued = 0;      // copy warp: packed stages issued (sequence count)
-    uint32_t mma_committed = 0;  // MMA warp: k-tiles committed (sequence count)
+    uint32_t mma_committed = 0;    // MMA warp: stages committed
+    bool single_changed = false;   // (kSingle) this thread saw a new bit
+    // Items, halves and operand stages are numbered through the CTA's work, by
+    // every role in the same way: slot or stage = number % count, use = number /
+    // count; a "full" barrier is waited with parity use & 1, an "empty" one with
+    // (use & 1) ^ 1 (a fresh barrier counts its previous phase as complete, so
+    // the first use passes).
 
-    bool single_changed = false;  // (kSingle) this thread saw a new bit
-    for (uint32_t round = 0;; ++round) {
-        if (!kSingle && tid == 0) S.item = atomicAdd(&st->item_next[2], 1u);
-        if (!kSingle) __syncthreads();
-        const uint32_t idx = kSingle ? blockIdx.x + round * gridDim.x : S.item;
-        if (idx >= nitems || *abort) break;
-        const uint64_t it = kSingle ? make_item(0, idx / single_blocks, idx % single_blocks, 0, single.a.T) : items[idx];
-        ProdDesc pd;
-        if (kSingle) {
-            pd.T = single.a.T;
-            pd.query = 0;
-            pd.head = 0;
-        } else {
-            pd = prods[item_prod(it)];
-        }
-        const uint32_t tig = item_ti(it), tjb = item_tjb(it), klo = item_klo(it), khi = item_khi(it);
-        const bool merged = !kSingle && (it & kItemMerged) != 0;
-        const DevMat P = kSingle ? single.a : resolve_operand(slots[pd.pslot], merged ? 0 : pd.p_delta, iter);
-        const DevMat Q = kSingle ? single.b : resolve_operand(slots[pd.qslot], merged ? 0 : pd.q_delta, iter);
-        const uint32_t *const dpocc = kSingle ? nullptr : slots[pd.pslot].dlt[iter & 1].occ;
-        const uint32_t *const dqocc = kSingle ? nullptr : slots[pd.qslot].dlt[iter & 1].occ;
-        const DevMat C = kSingle ? single.c : slots[pd.head].cur;
-        DevMat D;
-        if (kSingle) D.bits = nullptr;
-        else D = slots[pd.head].dlt[(iter & 1) ^ 1];
-        const uint32_t T = pd.T, ow = P.ow;
-        const uint32_t ti0 = tig * 4, tj0 = tjb * 4;
-        const uint32_t qword = tj0 >> 5, qshift = tj0 & 31;
-        const uint32_t np = min(4u, T - ti0), nq = min(4u, T - tj0);  // existing P tile-rows / Q tiles
-
-        // ---- k-list: tk with an occupied P tile in the 4 tile-rows and a
-        // non-empty Q block, increasing tk, within the item's range ----
-        if (warp == 0) {
-            uint32_t nc = 0;
-            for (uint32_t base = 0; base < ow; base += 32) {
-                uint32_t bits = 0;
-                if (base + lane < ow) {
-                    for (uint32_t g = 0; g < np; ++g) bits |= P.occ[(size_t)(ti0 + g) * ow + base + lane];
-                    bits &= range_word_mask(base + lane, klo, khi);
+    if (warp == kListWarp) {
+        const uint64_t *const items = items_all + 2 * list_cap;
+        const uint32_t blocks = (single.a.T + 3) / 4;
+        const uint32_t nitems = kSingle ? blocks * blocks : st->item_count[2];
+        uint32_t idx = kSingle ? blockIdx.x : 0u;
+        for (uint32_t posted = 0;;) {
+            // the next claim waits until the item before it is in its last half:
+            // a claim far ahead would take work from CTAs that are idle
+            if (posted && !warp_wait(&S.claim, (posted - 1) & 1u, abort)) break;
+            if (!warp_wait(&S.list_empty[posted & 1], ((posted >> 1) & 1u) ^ 1u, abort)) break;
+            ListSlot &L = S.list[posted & 1];
+            uint32_t nk[2] = {0, 0};
+            bool last = false;
+            for (;;) {  // items until one with k-tiles
+                if (!kSingle) {
+                    if (lane == 0) idx = atomicAdd(&st->item_next[2], 1u);
+                    idx = __shfl_sync(kFull, idx, 0);
                 }
-                const uint32_t cnt = __popc(bits);
-                uint32_t pre = cnt;
-#pragma unroll
-                for (int o = 1; o < 32; o <<= 1) {
-                    const uint32_t v = __shfl_up_sync(kFull, pre, o);
-                    if (lane >= (uint32_t)o) pre += v;
+                if (idx >= nitems || *abort) {
+                    last = true;
+                    break;
                 }
-                uint32_t pos = nc + pre - cnt;
-                while (bits) {
-                    S.cand[pos++] = (uint16_t)((base + lane) * 32 + (__ffs(bits) - 1));
-                    bits &= bits - 1;
+                const uint64_t it =
+                    kSingle ? make_item(0, idx / blocks, idx % blocks, 0, single.a.T) : items[idx];
+                if (kSingle) idx += gridDim.x;
+                ProdDesc pd;
+                if (kSingle) {
+                    pd.T = single.a.T;
+                    pd.query = 0;
+                    pd.head = 0;
+                } else {
+                    pd = prods[item_prod(it)];
                 }
-                nc += __shfl_sync(kFull, pre, 31);
-            }
-            if (lane == 0) S.nc = nc;
-        }
-        __syncthreads();
-        const uint32_t nc = S.nc, rounds = (nc + 31) / 32;
-        for (uint32_t r = warp; r < rounds; r += kThreads / 32) {
-            const uint32_t c = r * 32 + lane;
-            uint32_t mask = 0;
-            if (c < nc) {
-                const uint32_t tk = S.cand[c];
-                bool dp = !merged;  // delta bits in the P tiles
-                if (merged)
-                    for (uint32_t g = 0; g < np; ++g)
-                        dp = dp || ((dpocc[(size_t)(ti0 + g) * ow + (tk >> 5)] >> (tk & 31)) & 1u);
-                mask = ((dp ? Q.occ : dqocc)[(size_t)tk * ow + qword] >> qshift) & 0xFu;
-            }
-            const unsigned ball = __ballot_sync(kFull, mask != 0);
-            if (c < nc) S.cmask[c] = (uint16_t)mask;
-            if (lane == 0) S.rball[r] = ball;
-        }
-        __syncthreads();
-        if (warp == 0) {
-            uint32_t carry = 0;
-            for (uint32_t base = 0; base < rounds; base += 32) {
-                const uint32_t r = base + lane;
-                const uint32_t cnt = r < rounds ? __popc(S.rball[r]) : 0;
-                uint32_t pre = cnt;
-#pragma unroll
-                for (int o = 1; o < 32; o <<= 1) {
-                    const uint32_t v = __shfl_up_sync(kFull, pre, o);
-                    if (lane >= (uint32_t)o) pre += v;
-                }
-                if (r < rounds) S.roff[r] = carry + pre - cnt;
-                carry += __shfl_sync(kFull, pre, 31);
-            }
-        }
-        __syncthreads();
-        for (uint32_t c = tid; c < nc; c += kThreads) {
-            if (!S.cmask[c]) continue;
-            const uint32_t rank = S.roff[c >> 5] + __popc(S.rball[c >> 5] & ((1u << (c & 31)) - 1));
-            S.ktile[rank] = S.cand[c];  // keeps increasing tk order
-            triples += 16;
-        }
-        if (tid == 0) S.nk = rounds ? S.roff[rounds - 1] + __popc(S.rball[rounds - 1]) : 0u;
-        __syncthreads();
-        const uint32_t nk = S.nk;
-
-        // ---- pipeline over the item's k-tiles ----
-        if (warp == kCopyWarp) {
-            if (lane == 0) {
-                for (uint32_t e = 0; e < nk; ++e) {
-                    const uint32_t q = seq + e, s = q % kPkStages, use = q / kPkStages;
-                    if (!wait_or_abort(&S.pk_empty[s], (use & 1u) ^ 1u, abort)) {
-                        *abort = 1;
-                        break;
-                    }
-                    const uint32_t tk = S.ktile[e];
-                    mbar_arrive_expect_tx(&S.pk_full[s], (np + nq) * 512u);
-                    for (uint32_t g = 0; g < np; ++g)
-                        bulk_g2s(S.pk[s][g], P.bits + tile_offset(T, ti0 + g, tk), 512u, &S.pk_full[s]);
-                    bulk_g2s(S.pk[s][4], Q.bits + tile_offset(T, tk, tj0), nq * 512u, &S.pk_full[s]);
-                    ++pk_issued;
-                }
-            }
-        } else if (warp == kMmaWarp) {
-            if (lane == 0) {
-                for (uint32_t e = 0; e < nk; ++e) {
-                    const uint32_t q = seq + e, o = q % kOpStages, use = q / kOpStages;
-                    if (!wait_or_abort(&S.op_full[o], use & 1u, abort)) {
-                        *abort = 1;
-                        break;
-                    }
-                    tc_fence_after();
-                    const uint32_t abase = smem_addr(S.a[o]), bbase = smem_addr(S.b[o]);
-#pragma unroll
-                    for (uint32_t h = 0; h < 2; ++h) {      // accumulator h: operand rows 128h .. 128h+127
-#pragma unroll
-                        for (uint32_t kh = 0; kh < 2; ++kh) {  // K halves of 32 bytes
-                            const uint64_t ad = smem_desc(abase + h * 8192 + kh * 256, 128, 512);
-                            const uint64_t bd = smem_desc(bbase + kh * 4 * kBLbo, kBLbo, kBSbo);
-                            mma_i8(tmem + h * 256, ad, bd, (e > 0 || kh > 0) ? 1u : 0u);
+                const bool merged = !kSingle && (it & kItemMerged) != 0;
+                const DevMat P = kSingle ? single.a : resolve_operand(slots[pd.pslot], merged ? 0 : pd.p_delta, iter);
+                const DevMat Q = kSingle ? single.b : resolve_operand(slots[pd.qslot], merged ? 0 : pd.q_delta, iter);
+                const uint32_t *const dpocc = kSingle ? nullptr : slots[pd.pslot].dlt[iter & 1].occ;
+                const uint32_t *const dqocc = kSingle ? nullptr : slots[pd.qslot].dlt[iter & 1].occ;
+                const uint32_t T = pd.T, ow = P.ow, klo = item_klo(it), khi = item_khi(it);
+                const uint32_t ti0 = item_ti(it) * 4, tj0 = item_tjb(it) * 4;
+                const uint32_t qword = tj0 >> 5, qshift = tj0 & 31;
+                // k-lists: tk with an occupied P tile in the 4 tile-rows and a
+                // non-empty Q half, increasing tk, within the item's range; in a
+                // merged item, P or Q with delta bits there
+                nk[0] = nk[1] = 0;
+                for (uint32_t base = 0; base < ow; base += 32) {
+                    uint32_t pu = 0, du = 0;
+                    if (base + lane < ow) {
+                        for (uint32_t g = 0; g < min(4u, T - ti0); ++g) {
+                            pu |= P.occ[(size_t)(ti0 + g) * ow + base + lane];
+                            if (merged) du |= dpocc[(size_t)(ti0 + g) * ow + base + lane];
                         }
+                        pu &= range_word_mask(base + lane, klo, khi);
                     }
-                    mma_commit(&S.op_empty[o]);
-                    ++mma_committed;
-                }
-                if (nk && !*abort) mma_commit(&S.acc_full);  // completes after every MMA of the item
-            }
-        } else {
-            // expander warp w of group gp (k-tiles e with e % 2 == gp): P tile
-            // w (w < 4) or Q tile w - 4 (by rows, no transpose)
-            const uint32_t gp = warp / kGroupWarps, wr = warp % kGroupWarps;
-            const bool is_p = wr < 4;
-            const uint32_t g = is_p ? wr : wr - 4;
-            const bool present = g < (is_p ? np : nq);
-            for (uint32_t e = gp; e < nk; e += 2) {
-                const uint32_t q = seq + e, s = q % kPkStages, o = q % kOpStages;
-                // waits are warp-uniform: one lane giving up ends the whole warp's loop
-                if (!__all_sync(kFull, wait_or_abort(&S.pk_full[s], (q / kPkStages) & 1u, abort))) {
-                    if (lane == 0) *abort = 1;
-                    break;
-                }
-                if (wr == 0 && lane == 0) S.pk_seen[q & 1u] = q + 1;
-                uint64_t lo = 0, hi = 0;
-                if (present) {
-                    lo = S.pk[s][is_p ? g : 4 + g][lane];
-                    hi = S.pk[s][is_p ? g : 4 + g][lane + 32];
-                }
-                __syncwarp();
-                if (lane == 0) mbar_arrive(&S.pk_empty[s]);  // the packed stage may be refilled
-                if (!__all_sync(kFull, wait_or_abort(&S.op_empty[o], ((q / kOpStages) & 1u) ^ 1u, abort))) {
-                    if (lane == 0) *abort = 1;
-                    break;
-                }
-                if (present) {
-                    if (is_p) {
-                        store_row_k(S.a[o] + g * 4096, lane, lo);
-                        store_row_k(S.a[o] + g * 4096, lane + 32, hi);
-                    } else {
-                        store_row_mn(S.b[o], g, lane, lo);
-                        store_row_mn(S.b[o], g, lane + 32, hi);
-                    }
-                }
-                fence_proxy_async_smem();  // generic-proxy writes before the tensor core reads them
-                __syncwarp();
-                if (lane == 0) mbar_arrive(&S.op_full[o]);
-            }
-        }
-        seq += nk;
-        __syncthreads();
-        if (*abort) break;
-
-        // ---- epilogue (expander warps) ----
-        bool any_new = false;
-        if (nk > 0 && warp < kExpWarps) {
-            const bool acc_ok = __all_sync(kFull, wait_or_abort(&S.acc_full, items_done & 1u, abort));
-            if (!acc_ok && lane == 0) *abort = 1;
-            tc_fence_after();
-            if (acc_ok) {
-                uint32_t tile_new[2] = {0, 0};
-                const uint32_t h = (warp >> 2) & 1u, qq = warp & 3, half = warp >> 3;
-                const uint32_t m = 128 * h + 32 * qq + lane;  // output row within the 256-row block
-                const uint32_t ti = ti0 + (m >> 6), r = m & 63;
-#pragma unroll 1
-                for (uint32_t jh = 0; jh < 2; ++jh) {
-                    const uint32_t jt = 2 * half + jh;
-                    uint32_t a32[2];
+                    for (uint32_t w0 = 0; w0 < min(32u, ow - base); w0 += 4) {
+                        uint32_t mask[4];
 #pragma unroll
-                    for (int x = 0; x < 2; ++x) {
-                        uint32_t v[32];
-                        tmem_ld32(tmem + ((32 * qq) << 16) + h * 256 + jt * 64 + x * 32, v);
-                        uint32_t w = 0;
+                        for (uint32_t i = 0; i < 4; ++i) {
+                            const uint32_t pw = __shfl_sync(kFull, pu, w0 + i), dw = __shfl_sync(kFull, du, w0 + i);
+                            const uint32_t tk = (base + w0 + i) * 32 + lane;
+                            mask[i] = 0;
+                            if ((pw >> lane) & 1u)
+                                mask[i] = ((!merged || ((dw >> lane) & 1u) ? Q.occ : dqocc)[(size_t)tk * ow + qword] >>
+                                           qshift) & 0xFu;
+                        }
 #pragma unroll
-                        for (int c = 0; c < 32; ++c) w |= (uint32_t)(v[c] != 0) << c;
-                        a32[x] = w;
-                    }
-                    const uint64_t a = (uint64_t)a32[0] | ((uint64_t)a32[1] << 32);
-                    const uint32_t tj = tj0 + jt;
-                    uint32_t newcnt = 0;
-                    if (a && ti < T && tj < T) {
-                        ++outw;
-                        const size_t off = tile_offset(T, ti, tj) + r;
-                        unsigned long long *cw = reinterpret_cast<unsigned long long *>(C.bits + off);
-                        const uint64_t seen = __ldcg(cw);
-                        if (a & ~seen) {
-                            const uint64_t prev = atomicOr(cw, (unsigned long long)a);
-                            const uint64_t nw = a & ~prev;
-                            if (nw) {
-                                ++neww;
-                                newcnt = __popcll(nw);
-                                if (D.bits)
-                                    atomicOr(reinterpret_cast<unsigned long long *>(D.bits + off),
-                                             (unsigned long long)nw);
+                        for (uint32_t i = 0; i < 4; ++i) {
+#pragma unroll
+                            for (uint32_t h = 0; h < 2; ++h) {
+                                const bool take = (mask[i] >> (2 * h)) & 3u;
+                                const uint32_t ball = __ballot_sync(kFull, take);
+                                if (take)
+                                    L.ktile[h][nk[h] + __popc(ball & ((1u << lane) - 1))] =
+                                        (uint16_t)((base + w0 + i) * 32 + lane);
+                                nk[h] += __popc(ball);
                             }
                         }
                     }
-                    tile_new[jh] = __reduce_add_sync(kFull, newcnt);  // the warp's 32 rows share (ti, tj)
                 }
-                any_new = (tile_new[0] | tile_new[1]) != 0;
-                if (any_new && ti < T) {  // lane j: tile tj0 + 2 * half + j (populations, occupancy, counters)
-                    const uint32_t mine = lane == 0 ? tile_new[0] : lane == 1 ? tile_new[1] : 0u;
-                    tiles_gain(C, ti, tj0 + 2 * half, mine, cnts ? cnts + 3 * pd.head : nullptr);
-                    if (D.bits)
-                        tiles_gain(D, ti, tj0 + 2 * half, mine,
-                                   cnts ? cnts + 3 * pd.head + 1 + ((iter & 1) ^ 1) : nullptr);
+                if (!(nk[0] | nk[1])) continue;
+                __syncwarp();
+                if (lane < 2 * kUnit) {  // whole units: the last k-tile again
+                    const uint32_t h = lane / kUnit, n = nk[h], k = (n / kUnit) * kUnit + lane % kUnit;
+                    if (n && k >= n && n % kUnit) L.ktile[h][k] = L.ktile[h][n - 1];
                 }
+                if (lane == 0) {
+                    L.nk[0] = nk[0];
+                    L.nk[1] = nk[1];
+                    L.ti0 = ti0;
+                    L.tj0 = tj0;
+                    L.T = T;
+                    L.head = pd.head;
+                    L.query = pd.query;
+                    L.p = P.bits;
+                    L.q = Q.bits;
+                    L.c = kSingle ? single.c : slots[pd.head].cur;
+                    if (kSingle) L.d.bits = nullptr;
+                    else L.d = slots[pd.head].dlt[(iter & 1) ^ 1];
+                    triples += 8ULL * (nk[0] + nk[1]);
+                }
+                break;
             }
+            if (lane == 0) L.last = last;
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&S.list_full[posted & 1]);
+            if (last) break;
+            ++posted;
         }
-        if (nk > 0) ++items_done;
-        if (kSingle) {
-            single_changed = single_changed || any_new;
-        } else if (any_new && lane == 0) {
-            st->changed = 1u;
-            if (qchanged) qchanged[pd.query] = 1u;
+    } else if (warp == kMmaWarp) {
+        if (lane == 0) {
+            const uint64_t bdesc0 = smem_desc(smem_addr(S.b[0]), kBLbo, kBSbo);
+            uint32_t seq = 0, halves = 0;
+            bool ok = true;
+            for (uint32_t item = 0; ok; ++item) {
+                ok = wait_or_abort(&S.list_full[item & 1], (item >> 1) & 1u, abort);
+                if (!ok) break;
+                const ListSlot &L = S.list[item & 1];
+                if (L.last) break;
+                const uint32_t lasth = L.nk[1] ? 1u : 0u;
+                for (uint32_t half = 0; half < 2 && ok; ++half) {
+                    const uint32_t nk = L.nk[half];
+                    if (half == lasth) {
+                        mbar_arrive(&S.claim);
+                    }
+                    if (!nk) continue;
+                    ok = wait_or_abort(&S.acc_empty, (halves & 1u) ^ 1u, abort);
+                    if (!ok) break;
+                    tc_fence_after();
+                    for (uint32_t k0 = 0; k0 < nk; k0 += kKt, ++seq) {
+                        const uint32_t o = seq % kOpStages;
+                        ok = wait_or_abort(&S.op_full[o], (seq / kOpStages) & 1u, abort);
+                        if (!ok) break;
+                        tc_fence_after();
+                        const uint32_t kts = min(kKt, nk - k0);
+                        const uint64_t bd = bdesc0 + o * (kKt * kBTile >> 4);
+#pragma unroll
+                        for (uint32_t kt = 0; kt < kKt; ++kt) {
+                            if (kt >= kts) break;
+                            mma_fp4(tmem, tmem + kACol + o * kACols + kt * 8, bd + kt * (kBTile >> 4), tmem + kSfCol,
+                                    (k0 > 0 || kt > 0) ? 1u : 0u);
+                        }
+                        mma_commit(&S.op_empty[o]);
+                        ++mma_committed;
+                    }
+                    if (ok) mma_commit(&S.acc_full);  // completes after every MMA of the half
+                    ++halves;
+                }
+                if (ok) mbar_arrive(&S.list_empty[item & 1]);
+            }
+            if (!ok) *abort = 1;
         }
-        tc_fence_before();
-        __syncthreads();  // TMEM reads done before the next item's first MMA overwrites it
-        tc_fence_after();
-        if (*abort) break;
+        __syncwarp();
+    } else {
+        const bool is_a = warp < kBFirst;
+        const uint32_t gp = is_a ? warp / kAWarps : (warp - kBFirst) / kBWarps;
+        // A warp: Q tile g of the half, columns 32 hf .. of it, k-tiles kUnit sub ..
+        // of a stage; B warp: P tile g, all rows and k-tiles
+        const uint32_t wr = warp % 4, sub = (warp >> 2) & 1u, hf = wr & 1u;
+        const uint32_t g = is_a ? wr >> 1 : wr;
+        const Transposer transpose(lane);
+        uint8_t *const brow = S.b[0] + (8 * g + (lane >> 3)) * kBSbo + (lane & 7) * 16;
+        uint32_t seq = 0, halves = 0;
+        bool pending = false;           // a half of this warp waits for its epilogue
+        uint32_t pslot = 0, phalf = 0;  // its list slot and half
+        bool plast = false;             // it is the item's last
+        bool ok = true;
+        for (uint32_t item = 0; ok; ++item) {
+            ok = warp_wait(&S.list_full[item & 1], (item >> 1) & 1u, abort);
+            if (!ok) break;
+            ListSlot &L = S.list[item & 1];
+            const bool last = L.last != 0;
+            for (uint32_t half = 0; half < 2 && ok; ++half) {
+                // (an end of the claims is a half without k-tiles)
+                const uint32_t nk = last ? 0u : L.nk[half];
+                if (!nk && !last) continue;
+                const uint32_t steps = (nk + kKt - 1) / kKt;
+                const uint32_t T = L.T, tj0 = L.tj0 + 2 * half, ti0 = L.ti0;
+                const uint16_t *const ktile = L.ktile[half];
+                // the lane's rows of a k-tile: A first_row(lane) and 16 further of Q tile
+                // g, B lane and lane + 32 of P tile g
+                // (a tile beyond the matrix: its last one, whose results are not taken)
+                const uint32_t tile = is_a ? min(tj0 + g, T - 1) : min(ti0 + g, T - 1);
+                const char *const src = reinterpret_cast<const char *>(
+                    is_a ? L.q + (size_t)tile * 64 + Transposer::first_row(lane) : L.p + tile_offset(T, tile, 0) + lane) +
+                    (is_a ? 4 * hf : 0u);
+                const uint32_t stride = is_a ? T * 512u : 512u;
+                uint32_t ahead[kUnit][4];  // A: 32 columns of the two rows; B: both rows
+                uint32_t tks[kUnit];
+                const uint32_t kmax = nk ? (nk - 1) / kUnit * kUnit : 0u;
+                auto ktiles = [&](uint32_t k0) {  // (lists are padded to whole units)
+                    const uint2 t = *reinterpret_cast<const uint2 *>(ktile + min(k0, kmax));
+                    tks[0] = t.x & 0xffffu;
+                    tks[1] = t.x >> 16;
+                    tks[2] = t.y & 0xffffu;
+                    tks[3] = t.y >> 16;
+                };
+                auto load = [&](uint32_t i) {
+                    const char *const at = src + (uint64_t)tks[i] * stride;
+                    if (is_a) {
+                        ahead[i][0] = __ldca(reinterpret_cast<const uint32_t *>(at));
+                        ahead[i][1] = __ldca(reinterpret_cast<const uint32_t *>(at + 16 * 8));
+                    } else {
+                        const uint2 u = __ldcg(reinterpret_cast<const uint2 *>(at));
+                        const uint2 v = __ldcg(reinterpret_cast<const uint2 *>(at + 32 * 8));
+                        ahead[i][0] = u.x;
+                        ahead[i][1] = u.y;
+                        ahead[i][2] = v.x;
+                        ahead[i][3] = v.y;
+                    }
+                };
+                if (nk) {
+                    ktiles(gp * kKt + (is_a ? sub * kUnit : 0u));
+#pragma unroll
+                    for (uint32_t i = 0; i < kUnit; ++i) load(i);
+                }
+                for (uint32_t e = gp;; e += 2) {
+                    if (e < steps) {
+                        const uint32_t q = seq + e, o = q % kOpStages, kts = min(kKt, nk - e * kKt);
+                        ok = warp_wait(&S.op_empty[o], ((q / kOpStages) & 1u) ^ 1u, abort);
+                        if (!ok) break;
+                        if (is_a) {
+                            tc_fence_after();
+                            if (sub * kUnit < kts) {
+                                uint32_t r[8 * kUnit];
+                                transpose(ahead);
+#pragma unroll
+                                for (uint32_t i = 0; i < kUnit; ++i) expand64(ahead[i][0], ahead[i][1], r + 8 * i);
+                                tmem_st32(tmem + ((32 * wr) << 16) + kACol + o * kACols + sub * kUnit * 8, r);
+                                ktiles((e + 2) * kKt + sub * kUnit);
+#pragma unroll
+                                for (uint32_t i = 0; i < kUnit; ++i) load(i);
+                                asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+                            }
+                            tc_fence_before();
+                        } else {
+                            uint8_t *const at = brow + o * kKt * kBTile;
+#pragma unroll
+                            for (uint32_t u = 0; u < kKt; u += kUnit) {
+                                if (u >= kts) break;
+                                ktiles(u + kUnit < kts ? e * kKt + u + kUnit : (e + 2) * kKt);
+#pragma unroll
+                                for (uint32_t i = 0; i < kUnit; ++i) {
+#pragma unroll
+                                    for (uint32_t j = 0; j < 2; ++j) {
+                                        uint32_t r[8];
+                                        expand64(ahead[i][2 * j], ahead[i][2 * j + 1], r);
+                                        uint8_t *const to = at + (u + i) * kBTile + 4 * j * kBSbo;
+                                        *reinterpret_cast<uint4 *>(to) = make_uint4(r[0], r[1], r[2], r[3]);
+                                        *reinterpret_cast<uint4 *>(to + kBLbo) = make_uint4(r[4], r[5], r[6], r[7]);
+                                    }
+                                    load(i);
+                                }
+                            }
+                            fence_proxy_async_smem();  // generic-proxy writes before the tensor core reads them
+                        }
+                        __syncwarp();
+                        if (lane == 0) mbar_arrive(&S.op_full[o]);
+                    }
+                    if (pending) {
+                        // ---- epilogue of the half before (number halves - 1) ----
+                        pending = false;
+                        const ListSlot &E = S.list[pslot];
+                        const uint32_t buf = (halves - 1) & 1u, qq = warp & 3, pg = warp >> 2;
+                        ok = warp_wait(&S.acc_full, buf, abort);
+                        if (!ok) break;
+                        tc_fence_after();
+#pragma unroll
+                        for (uint32_t x = 0; x < 2; ++x) {  // column of the half 32 qq + lane, rows 64 pg + 32 x ..
+                            uint32_t v[32];
+                            tmem_ld32(tmem + ((32 * qq) << 16) + pg * 64 + x * 32, v);
+                            uint32_t w = 0;
+#pragma unroll
+                            for (int c = 0; c < 32; ++c) w = __funnelshift_l(__float_as_uint(0.0f - __uint_as_float(v[31 - c])), w, 1);
+                            S.out[buf][qq][pg * 64 + x * 32 + lane] = transpose32(w, lane);
+                        }
+                        tc_fence_before();
+                        __syncwarp();
+                        if (lane == 0) mbar_arrive(&S.acc_empty);  // the accumulator may be overwritten
+                        ok = warp_wait(&S.acc_empty, buf, abort);  // every warp's bits are there
+                        if (!ok) break;
+                        const uint32_t jt = (warp >> 1) & 1u, r = (warp & 1u) * 32 + lane;
+                        const uint32_t ti = E.ti0 + pg, tj = E.tj0 + 2 * phalf + jt;
+                        const uint64_t a = (uint64_t)S.out[buf][2 * jt][pg * 64 + r] |
+                                           ((uint64_t)S.out[buf][2 * jt + 1][pg * 64 + r] << 32);
+                        uint32_t newcnt = 0;
+                        if (a && ti < E.T && tj < E.T) {
+                            ++outw;
+                            const size_t off = tile_offset(E.T, ti, tj) + r;
+                            unsigned long long *cw = reinterpret_cast<unsigned long long *>(E.c.bits + off);
+                            const uint64_t seen = __ldcg(cw);
+                            if (a & ~seen) {
+                                const uint64_t prev = atomicOr(cw, (unsigned long long)a);
+                                const uint64_t nw = a & ~prev;
+                                if (nw) {
+                                    ++neww;
+                                    newcnt = __popcll(nw);
+                                    if (E.d.bits)
+                                        atomicOr(reinterpret_cast<unsigned long long *>(E.d.bits + off),
+                                                 (unsigned long long)nw);
+                                }
+                            }
+                        }
+                        const uint32_t tile_new = __reduce_add_sync(kFull, newcnt);  // 32 rows of one tile
+                        if (tile_new) {  // lane 0: tile tj (populations, occupancy, counters)
+                            const uint32_t mine = lane == 0 ? tile_new : 0u;
+                            tiles_gain(E.c, ti, tj, mine, cnts ? cnts + 3 * E.head : nullptr);
+                            if (E.d.bits)
+                                tiles_gain(E.d, ti, tj, mine, cnts ? cnts + 3 * E.head + 1 + ((iter & 1) ^ 1) : nullptr);
+                            if (kSingle) {
+                                single_changed = true;
+                            } else if (lane == 0) {
+                                st->changed = 1u;
+                                if (qchanged) qchanged[E.query] = 1u;
+                            }
+                        }
+                        __syncwarp();
+                        if (plast && lane == 0) mbar_arrive(&S.list_empty[pslot]);
+                    }
+                    if (e + 2 >= steps) break;
+                }
+                if (!nk || !ok) break;
+                seq += steps;
+                ++halves;
+                const bool final_half = half == 1 || !L.nk[1];
+                if (warp < kEpiWarps) {
+                    pending = true;
+                    pslot = item & 1;
+                    phalf = half;
+                    plast = final_half;
+                } else if (final_half) {
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(&S.list_empty[item & 1]);
+                }
+                if (final_half) break;  // the slot may already hold another item
+            }
+            if (last) break;
+        }
     }
 
-    // ---- exit: after a wait gave up, wait (bounded) for every bulk copy and
-    // MMA still in flight before TMEM is freed and the CTA ends ----
+    // ---- exit: after a wait gave up, wait (bounded) for every MMA still in
+    // flight before TMEM is freed and the CTA ends ----
     __syncthreads();
     const bool aborted = *abort != 0;
-    if (aborted) {
-        if (warp == kCopyWarp && lane == 0) {
-            // copies of the stages not seen by their group may still be
-            // landing (a stage is refilled only after its group saw it)
-            const uint32_t seen0 = S.pk_seen[0], seen1 = S.pk_seen[1];
-            for (uint32_t q = min(seen0, seen1); q < pk_issued; ++q)
-                if (q >= ((q & 1u) ? seen1 : seen0)) mbar_wait_bounded(&S.pk_full[q % kPkStages], (q / kPkStages) & 1u);
-        }
-        if (warp == kMmaWarp && lane == 0 && mma_committed) {
-            // the last commit completes after every MMA issued before it
-            const uint32_t q = mma_committed - 1;
-            mbar_wait_bounded(&S.op_empty[q % kOpStages], (q / kOpStages) & 1u);
-        }
+    if (aborted && warp == kMmaWarp && lane == 0 && mma_committed) {
+        // the last commit completes after every MMA issued before it
+        const uint32_t q = mma_committed - 1;
+        mbar_wait_bounded(&S.op_empty[q % kOpStages], (q / kOpStages) & 1u);
     }
     if (kSingle) {
         const bool changed = __syncthreads_or(single_changed) != 0;
