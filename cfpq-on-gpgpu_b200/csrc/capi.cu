@@ -70,6 +70,9 @@ constexpr uint32_t kLeaveItems = 12;
 // 1464.  AUTO at n = 12000 keeps the launch for its tensor cores: dense 1573 us
 // against 4556 with LOP3.
 constexpr uint32_t kAddMulMaxTiles = 256;
+// The device's choice between them costs two launches, 8 us: worth it from n =
+// 2048 on (dense: LOP3 45 us, tensor cores 31; 26 and 27 at n = 1024).
+constexpr uint32_t kAddMulMinTcTiles = 32;
 constexpr uint32_t kAddMulMaxWordTiles = 128;
 // Slots of the context's pinned flag block that receive a single product's
 // changed and error words.
@@ -1005,10 +1008,11 @@ static int add_mul_impl(cfpq_ctx *ctx, cfpq_matrix *c, const cfpq_matrix *a, con
     if (c->d.n == 0) return CFPQ_OK;
     // AUTO: tensor cores or LOP3 by the selector's rule, decided on the device
     // right before the product (choose, LOP3 and tensor-core launches, the one
-    // not chosen returns at once); below the tensor cores' size, LOP3
+    // not chosen returns at once); below kAddMulMinTcTiles or the selector's
+    // size, LOP3
     const bool choose = variant == CFPQ_VARIANT_AUTO && ctx->sel.mode != CFPQ_SELECT_FIXED && ctx->tc_grid &&
                         (ctx->sel.allowed & (1u << CFPQ_VARIANT_TC)) && ctx->h_flag_dev &&
-                        c->d.T >= ctx->sel.tc_min_tiles && c->d.T <= kAddMulMaxTiles;
+                        c->d.T >= std::max(ctx->sel.tc_min_tiles, kAddMulMinTcTiles) && c->d.T <= kAddMulMaxTiles;
     if (variant == CFPQ_VARIANT_AUTO) variant = CFPQ_VARIANT_LOP3;
     const bool alias = (a == c) || (b == c);
     if (variant == CFPQ_VARIANT_PLAIN) {

@@ -10,18 +10,18 @@ void selector_defaults(SelectorParams *sp) {
     memset(sp, 0, sizeof(*sp));
     sp->mode = CFPQ_SELECT_HEURISTIC;
     sp->allowed = (1u << CFPQ_VARIANT_LOP3) | (1u << CFPQ_VARIANT_M4R) | (1u << CFPQ_VARIANT_TC);
-    // Until cfpq_autotune runs: tensor cores for n >= 1024 when a fifth of
-    // the P tiles are occupied and 30% of them dense (fit to the exhaustive
-    // per-term timings of a chain closure at n = 32768; the size from whole
-    // closures, whose tensor-core terms share one plan and one product launch
-    // per iteration: limits of 32, 16 and 8 tiles give 17.6, 16.1 and 16.0 ms
-    // for 40 mixed queries, 1205, 995 and 968 us for a random CNF at n = 1200,
-    // 1831, 1600 and 1634 us at n = 1800); Four Russians when a quarter of the
-    // P tiles are dense.  (A single query selects from n >= 64 * min_tiles,
+    // Until cfpq_autotune runs: tensor cores for n >= 768 when a tenth of the P
+    // tiles are occupied and 10% of them dense (dense_tile_pop).  Measured on
+    // whole closures, whose tensor-core terms share one plan and one product
+    // launch per iteration: sizes from 16, 12 and 8 tiles on give 13.2, 12.4 and
+    // 12.2 ms for 40 mixed queries, 1225, 1247 and 1233 us for a random CNF at n =
+    // 1800; shares of 0.3 at 0.2 occupied and 0.15 at 0.1 give 279 and 260 ms
+    // for the chain closure at n = 16384 (tiles of more than 16 bits).  Four
+    // Russians when a quarter of the P tiles are dense.  (A single query selects from n >= 64 * min_tiles,
     // and below once its iterations are heavy.)
-    sp->tc_min_tiles = 16;
-    sp->tc_min_occ = 0.2f;
-    sp->tc_min_dense = 0.3f;
+    sp->tc_min_tiles = kTcTiles;
+    sp->tc_min_occ = 0.1f;
+    sp->tc_min_dense = 0.1f;
     sp->m4r_min_dense = 0.25f;
     sp->conf_margin = 0.05f;
     sp->range_margin = 0.1f;

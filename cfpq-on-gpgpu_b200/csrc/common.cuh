@@ -109,14 +109,27 @@ struct MatRows {
 // Statistics of one buffer of a closure (a slot's current matrix or one of
 // its two deltas), kept exact by the product epilogues and reset when a delta
 // is cleared: population, occupied tiles (occupancy bits), dense tiles
-// (population > kDenseTilePop).  Buffer b of slot s is counters[3*s + b]
+// (population > dense_tile_pop(T)).  Buffer b of slot s is counters[3*s + b]
 // (b = 0: current matrix, 1 + d: delta d).  They are the selector's features.
 struct BufCounters {
     unsigned long long nnz;
     uint32_t occ_tiles;
     uint32_t dense_tiles;
 };
-constexpr uint32_t kDenseTilePop = 96;
+// A tile counts as dense from the population on at which the cheaper of the
+// word-level kernels loses to the variant that would take its product.  Sizes
+// that the tensor cores take (kTcTiles..2048 tiles): more than kTcTilePop bits.
+// A k-tile costs them the same whatever it holds; by itself a product at n =
+// 8192 breaks even at 8 bits a tile (257 against 242 us; 257 against 560 at 82),
+// and in a closure, whose tiles fill up within an iteration, earlier: limits of
+// 96, 40, 16, 8 and 4 bits give 313, 287, 262, 253 and 230 ms for the chain closure
+// at n = 16384, 3.37, 3.21, 2.40, 2.42 and 2.12 ms for a random CNF at n = 3001.
+// Elsewhere Four Russians are the alternative, ahead only above kDenseTilePop
+// (560 us for LOP3 against 800 at 82 bits, 1400 against 935 at 1200).
+constexpr uint32_t kDenseTilePop = 96, kTcTilePop = 4, kTcTiles = 12;
+__host__ __device__ constexpr uint32_t dense_tile_pop(uint32_t T) {
+    return T >= kTcTiles && T <= 2048 ? kTcTilePop : kDenseTilePop;
+}
 
 // Variant selector (device-resident).  Feature vector of a product term,
 // predicted log-microseconds per candidate variant (LOP3, M4R, TC).
@@ -353,6 +366,7 @@ __device__ __forceinline__ void tiles_gain(const DevMat &m, uint32_t ti, uint32_
     const uint32_t lane = threadIdx.x & 31;
     const uint32_t tj = tj0 + lane;
     uint32_t gained = 0, dense = 0;
+    const uint32_t limit = dense_tile_pop(m.T);
     if (lane < 4 && add) {
         const size_t t = (size_t)ti * m.T + tj;
         const uint32_t bit = 1u << (tj & 31);
@@ -360,7 +374,7 @@ __device__ __forceinline__ void tiles_gain(const DevMat &m, uint32_t ti, uint32_
             const uint32_t old_pop = atomicAdd(m.nnz + t, add);
             const uint32_t old_occ = atomicOr(m.occ + (size_t)ti * m.ow + (tj >> 5), bit);
             gained = (old_occ & bit) ? 0u : 1u;
-            dense = (old_pop <= kDenseTilePop && old_pop + add > kDenseTilePop) ? 1u : 0u;
+            dense = (old_pop <= limit && old_pop + add > limit) ? 1u : 0u;
         } else {
             atomicAdd(m.nnz + t, add);
             atomicOr(m.occ + (size_t)ti * m.ow + (tj >> 5), bit);

@@ -21,7 +21,7 @@
 //   0 log2 n / 17            1 term (0: dA*B, 1: A*dB)
 //   2 P occupied-tile frac   3 Q occupied-tile frac
 //   4 P mean tile population / 4096          5 same for Q
-//   6 P dense-tile fraction (population > 96 of occupied)   7 same for Q
+//   6 P dense-tile fraction (population > dense_tile_pop(T)) of occupied   7 same for Q
 //   8 log2(1 + nnz P) / 34   9 log2(1 + nnz Q) / 34
 //  10 nnz of the delta operand / nnz of its slot's current matrix
 //  11 log2(1 + occP * occQ / T) / 32  (expected tile triples, uniform tiles)
@@ -70,10 +70,11 @@ __global__ void k_counters_init(const MatSlot *__restrict__ slots, BufCounters *
     unsigned long long nnz = 0;
     uint32_t occ = 0, dense = 0;
     const size_t tiles = (size_t)m.T * m.T, words = (size_t)m.T * m.ow;
+    const uint32_t limit = dense_tile_pop(m.T);
     for (size_t i = threadIdx.x; i < tiles; i += blockDim.x) {
         const uint32_t pop = m.nnz[i];
         nnz += pop;
-        dense += pop > kDenseTilePop;
+        dense += pop > limit;
     }
     for (size_t i = threadIdx.x; i < words; i += blockDim.x) occ += __popc(m.occ[i]);
     __shared__ unsigned long long s_nnz[32];
@@ -106,11 +107,15 @@ __global__ void k_counters_init(const MatSlot *__restrict__ slots, BufCounters *
 }
 
 // Variant of one product by itself (cfpq_add_mul with AUTO): the heuristic's
-// tensor-core rule on the left operand's tile statistics.  One block.
+// tensor-core rule on the left operand's tile statistics, with tiles of more
+// than 16 bits as the dense ones: the operands do not fill up as in a closure,
+// and at n = 8192 LOP3 takes 242 us at 8 bits a tile and 560 at 82, the tensor
+// cores 257.  One block.
+constexpr uint32_t kAddMulTilePop = 16;
 __global__ void __launch_bounds__(1024) k_add_mul_choose(DevMat a, float min_occ, float min_dense, uint32_t *use_tc) {
     const uint32_t tiles = a.T * a.T, words = a.T * a.ow;
     uint32_t occ = 0, dense = 0;
-    for (uint32_t i = threadIdx.x; i < tiles; i += blockDim.x) dense += a.nnz[i] > kDenseTilePop;
+    for (uint32_t i = threadIdx.x; i < tiles; i += blockDim.x) dense += a.nnz[i] > kAddMulTilePop;
     for (uint32_t i = threadIdx.x; i < words; i += blockDim.x) occ += __popc(a.occ[i]);
     occ = __reduce_add_sync(kFull, occ);
     dense = __reduce_add_sync(kFull, dense);
