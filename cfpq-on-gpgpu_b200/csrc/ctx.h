@@ -151,6 +151,9 @@ struct cfpq_ctx {
     std::vector<MatRows> clear_tab;    // matrix list of the clear in flight, sent in its launch
     void *h_edges = nullptr;           // pinned block of short pageable edge lists (kEdgeStageBytes)
     uint32_t *h_edges_dev = nullptr;   // the same as the device sees it
+    void *h_rows = nullptr;            // pinned halves that rows on their way to pageable memory pass (kRowStageBytes)
+    uint64_t *h_rows_dev = nullptr;    // the same as the device sees it
+    cudaEvent_t rows_done[2] = {nullptr, nullptr};  // a half's rows have arrived
     std::vector<unsigned char> edge_tables_key;  // large tables of the last edge load still in edge_buf
     std::vector<unsigned char> clear_desc_key;   // matrix list of the last cfpq_matrices_clear in clear_desc
     std::vector<unsigned char> diag_desc_key;    // epsilon matrices of the last cfpq_intersection in diag_desc

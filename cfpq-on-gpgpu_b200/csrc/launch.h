@@ -35,7 +35,8 @@ cudaError_t launch_ntset_unpack(const void *cells, uint32_t stride, uint32_t nma
 cudaError_t launch_ntset_square(void *cells, uint32_t n, uint32_t stride, uint32_t nmats, const void *d_rules,
                                 uint32_t nrules, uint32_t ymask, uint32_t *counters, int num_sms, cudaStream_t s);
 cudaError_t launch_rows_to_tiles(const DevMat &m, const uint64_t *d_rows, cudaStream_t s);
-cudaError_t launch_tiles_to_rows(const DevMat &m, uint64_t *d_rows, cudaStream_t s);
+// Rows row0 .. row0 + nrows - 1 in row-major words (vertex order) to d_rows.
+cudaError_t launch_tiles_to_rows(const DevMat &m, uint64_t *d_rows, uint32_t row0, uint32_t nrows, cudaStream_t s);
 cudaError_t launch_copy_matrix(const DevMat &dst, const DevMat &src, cudaStream_t s);
 cudaError_t launch_clear_matrix(const DevMat &m, cudaStream_t s);
 // Seeded random matrix with the given bit density (not for ordered matrices).
