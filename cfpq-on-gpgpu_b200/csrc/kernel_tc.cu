@@ -340,7 +340,11 @@ __global__ void __launch_bounds__(kThreads, 1)
     // every role in the same way: slot or stage = number % count, use = number /
     // count; a "full" barrier is waited with parity use & 1, an "empty" one with
     // (use & 1) ^ 1 (a fresh barrier counts its previous phase as complete, so
-    // the first use passes).
+    // the first use passes).  A wait by parity must not come two phases early:
+    // the groups take the stages by the parity of their number, not of their
+    // place in the half, so that a group's wait for stage q - 2 (the MMAs of q - 5
+    // are done) bounds its next one, for the MMAs of q - 3, in a row of halves
+    // of one stage too.
 
     if (warp == kListWarp) {
         const uint64_t *const items = items_all + 2 * list_cap;
@@ -517,7 +521,7 @@ __global__ void __launch_bounds__(kThreads, 1)
                 // (an end of the claims is a half without k-tiles)
                 const uint32_t nk = last ? 0u : L.nk[half];
                 if (!nk && !last) continue;
-                const uint32_t steps = (nk + kKt - 1) / kKt;
+                const uint32_t steps = (nk + kKt - 1) / kKt, first = (gp ^ seq) & 1u;  // group gp: stages of that number parity
                 const uint32_t T = L.T, tj0 = L.tj0 + 2 * half, ti0 = L.ti0;
                 const uint16_t *const ktile = L.ktile[half];
                 // the lane's rows of a k-tile: A first_row(lane) and 16 further of Q tile
@@ -553,11 +557,11 @@ __global__ void __launch_bounds__(kThreads, 1)
                     }
                 };
                 if (nk) {
-                    ktiles(gp * kKt + (is_a ? sub * kUnit : 0u));
+                    ktiles(first * kKt + (is_a ? sub * kUnit : 0u));
 #pragma unroll
                     for (uint32_t i = 0; i < kUnit; ++i) load(i);
                 }
-                for (uint32_t e = gp;; e += 2) {
+                for (uint32_t e = first;; e += 2) {
                     if (e < steps) {
                         const uint32_t q = seq + e, o = q % kOpStages, kts = min(kKt, nk - e * kKt);
                         ok = warp_wait(&S.op_empty[o], ((q / kOpStages) & 1u) ^ 1u, abort);

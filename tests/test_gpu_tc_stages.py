@@ -36,3 +36,30 @@ def test_tc_partial_stages(ctx, tiles, columns):
         finally:
             for m in (ma, mb, mc):
                 m.destroy()
+
+
+@pytest.mark.parametrize("seed", range(4))
+def test_tc_rows_of_short_halves(ctx, seed):
+    """Many items a CTA whose halves take one, two or no stages in any order: a
+    group of expanders that has no stage in a row of halves must not run ahead."""
+    tiles, rng = 150, np.random.default_rng(seed)
+    n = 64 * tiles
+    occupied = rng.random((tiles, tiles), dtype=np.float32) < rng.choice([0.005, 0.02, 0.06], tiles)[:, None]
+    a = np.zeros((n, n), dtype=bool)
+    for ti, tk in zip(*np.nonzero(occupied)):
+        a[64 * ti + rng.integers(0, 64, 8), 64 * tk + rng.integers(0, 64, 8)] = True
+    b = (rng.random((n, n), dtype=np.float32) < 0.01) & np.repeat(np.repeat(
+        rng.random((tiles, tiles), dtype=np.float32) < 0.5, 64, axis=0), 64, axis=1)
+    ma, mb, mc, want = (ctx.matrix(n) for _ in range(4))
+    try:
+        ma.upload_rows(_pack(a))
+        mb.upload_rows(_pack(b))
+        ctx.add_mul(want, ma, mb, "lop3")
+        rows = want.download_rows()
+        for _ in range(10):
+            mc.clear()
+            ctx.add_mul(mc, ma, mb, "tc")
+            assert np.array_equal(mc.download_rows(), rows)
+    finally:
+        for m in (ma, mb, mc, want):
+            m.destroy()
