@@ -16,8 +16,9 @@
 // (cp.async.bulk, the TMA engine) completing on an mbarrier, four k-tiles in flight,
 // and the CTA runs one of three inner loops on the staged tiles, chosen by the
 // population of the P tile:
-//   dense  (population > kSparseMax), all kBJ Q tiles staged (one contiguous
-//          range of the tiled layout, empty tiles are zeros):
+//   dense  (population > kSparseMaxLop3, kSparseMaxM4R), all kBJ Q tiles
+//          staged (one contiguous range of the tiled layout, empty tiles are
+//          zeros):
 //          LOP3: per row and inner index k, mask = -(P[row] bit k) (2 ALU
 //          ops), then acc |= mask & Q[k] on 8 uint32 words (one LOP3 each); Q
 //          rows k, k+1 of a tile come in one 16-byte shared load read by all
@@ -27,11 +28,11 @@
 //          (a table row per key, padded to 17 words so that lanes reading
 //          different keys hit different banks); each row then ORs one table
 //          word per slab and tile: 16 loads instead of 64 masked LOP3s.
-//   sparse (population <= kSparseMax), only the range of occupied Q tiles
-//          staged: a thread walks up to kLaneBits set bits k of each of its
-//          two P rows and ORs row k of each occupied Q tile of its warp from
-//          shared memory; the bits left in rows of hub vertices are spread
-//          over the warp's lanes one row at a time and OR-reduced.
+//   sparse (the others), only the range of occupied Q tiles
+//          staged: a thread walks the set bits k of its two P rows and ORs row
+//          k of each occupied Q tile of its warp from shared memory; rows of
+//          hub vertices, when few are left, are done by the whole warp one at
+//          a time and OR-reduced.
 // A warp skips its empty Q tiles (all of them: no inner loop at all).
 //
 // Epilogue: for each non-zero accumulator word, new = acc & ~old via a 64-bit

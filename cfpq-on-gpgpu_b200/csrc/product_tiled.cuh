@@ -12,10 +12,15 @@ namespace tiled {
 
 constexpr int kBJ = 16;              // output tiles per work item (1024 columns)
 constexpr uint32_t kStages = 4;      // staged k-tiles in flight per CTA (product kernels)
-constexpr uint32_t kLaneBits = 4;    // sparse loop: bits per row a lane walks before the warp helps
+constexpr uint32_t kLaneBits = 4;    // sparse loop: bits per row a lane walks at a time
+constexpr uint32_t kHelpRows = 2;    // ... and the bits in whose time the warp does one row together
 constexpr int kThreads = 128;        // 4 warps (product kernels; the persistent kernel runs 8)
 constexpr int kMaxTiles = 2048;      // k-list capacity (n <= 131072)
-constexpr uint32_t kSparseMax = 96;  // P-tile population up to which the sparse loop runs
+// P-tile population up to which the sparse loop runs.  Products at n = 5000 with
+// random bits, LOP3 loop: 82 bits a tile 119 us, 205 bits 173 against 376 in the
+// dense loop, 410 bits 244 against 392, 819 bits 361 dense; Four Russians 205
+// bits 215 against 277, 410 bits 300 against 256.
+constexpr uint32_t kSparseMaxLop3 = 512, kSparseMaxM4R = 256;
 constexpr int kTabRow = 17;          // padded table row (uint64 words): 16 keys, or kBJ tiles
 constexpr unsigned kFull = 0xffffffffu;
 constexpr uint32_t kGateSpinLimit = 1u << 24;  // ~1 s of polling
@@ -47,21 +52,6 @@ __device__ __forceinline__ DevMat resolve_operand(const MatSlot &s, uint8_t use_
 __device__ __forceinline__ uint32_t bitmask(uint32_t word, int b) {
     // all-ones if bit b of word is set, else zero
     return (uint32_t)((int32_t)(word << (31 - b)) >> 31);
-}
-
-// Position of the n-th (0-based) set bit of x (x has more than n set bits).
-__device__ __forceinline__ uint32_t nth_bit(uint32_t x, uint32_t n) {
-    uint32_t pos = 0;
-#pragma unroll
-    for (uint32_t s = 16; s > 0; s >>= 1) {
-        const uint32_t c = __popc(x & ((1u << s) - 1));
-        if (n >= c) {
-            n -= c;
-            x >>= s;
-            pos += s;
-        }
-    }
-    return pos;
 }
 
 __device__ __forceinline__ void or64(uint2 &a, uint64_t v) {
@@ -100,6 +90,7 @@ __device__ __forceinline__ void process_item(Smem &S, uint64_t it, const ProdDes
     constexpr uint32_t kNT = 32u * kW;         // threads
     constexpr uint32_t kWMask = (1u << kTPW) - 1;
     constexpr uint32_t kSt = Smem::kNumStages;       // staged k-tiles in flight
+    constexpr uint32_t kAtOnce = kTPW <= 2 ? 2 : 1;  // sparse loop: bits of a row whose Q words load together
     static_assert(kSt <= 32, "one mbarrier parity bit per stage");
     const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     unsigned long long &triples = ctr.triples, &staged = ctr.staged, &outw = ctr.outw, &neww = ctr.neww;
@@ -137,7 +128,7 @@ __device__ __forceinline__ void process_item(Smem &S, uint64_t it, const ProdDes
             const uint32_t pn = P.nnz[(size_t)ti * T + tk];
             if ((pw >> (tk & 31)) & 1u) {
                 mask = (qw >> qshift) & ((1u << kBJ) - 1);
-                dense = pn > kSparseMax;
+                dense = pn > (kM4R ? kSparseMaxM4R : kSparseMaxLop3);
             }
         }
         const unsigned ball = __ballot_sync(kFull, mask != 0);
@@ -194,7 +185,7 @@ __device__ __forceinline__ void process_item(Smem &S, uint64_t it, const ProdDes
             const uint32_t tk = S.cand[c];
             const bool dp = !merged || ((dpocc[(size_t)ti * ow + (tk >> 5)] >> (tk & 31)) & 1u);
             mask = ((dp ? Q.occ : dqocc)[(size_t)tk * ow + qword] >> qshift) & ((1u << kBJ) - 1);
-            dense = P.nnz[(size_t)ti * T + tk] > kSparseMax;  // issued together with the occupancy load
+            dense = P.nnz[(size_t)ti * T + tk] > (kM4R ? kSparseMaxM4R : kSparseMaxLop3);  // issued together with the occupancy load
         }
         const unsigned ball = __ballot_sync(kFull, mask != 0);
         if (c < nc) {
@@ -272,61 +263,79 @@ __device__ __forceinline__ void process_item(Smem &S, uint64_t it, const ProdDes
         const uint4 pp = *reinterpret_cast<const uint4 *>(&S.p[stage][2 * lane]);
         const bool dense = (S.ktile[e] & 0x8000u) != 0;
         if (!dense) {
-            // sparse P tile, only the occupied Q tiles staged.  Each lane
-            // first walks up to kLaneBits set bits of its rows 2l and 2l+1;
-            // the bits left (rows of hub vertices) are then handled one row
-            // at a time by the whole warp: lane i takes the i-th remaining
-            // bit, and the partial ORs meet in a warp OR-reduction.
+            // sparse P tile, only the occupied Q tiles staged.  Either each lane
+            // walks the set bits of its rows 2l and 2l+1, kLaneBits at a time,
+            // or, when few rows have many bits left (rows of hub vertices), the
+            // warp takes them one row at a time: lane i the Q rows i and i +
+            // 32, and the partial ORs meet in warp reductions.  What bounds it
+            // is latency: often one warp alone has occupied Q tiles, and the
+            // others wait for it.  So the Q words of both rows and kAtOnce bits
+            // load together (a word at a time cost ~200 clocks a bit), a row
+            // done together costs two reductions per tile (five shuffle steps
+            // before, ~700 clocks), and many rows with a few bits more than
+            // kLaneBits are walked on.  Same-generation at n = 8192: items of
+            // two such tiles 8-9 us -> 5-6, the call 403 -> 383 us; 35 products
+            // of the worklist at n = 777 880 -> 838 us.
             if (wmask && !timed_out) {
                 const uint64_t *q = &S.q[stage][(kTPW * warp) * 64];
                 uint64_t xa = ((uint64_t)pp.y << 32) | pp.x;
                 uint64_t xb = ((uint64_t)pp.w << 32) | pp.z;
 #pragma unroll 1
-                for (uint32_t it = 0; it < kLaneBits && (xa | xb); ++it) {
-                    if (xa) {
-                        const int k = __ffsll((long long)xa) - 1;
-                        xa &= xa - 1;
+                for (;;) {
+#pragma unroll 1
+                    for (uint32_t i = 0; i < kLaneBits && (xa | xb); i += kAtOnce) {
+                        uint2 va[kAtOnce][kTPW], vb[kAtOnce][kTPW];
 #pragma unroll
-                        for (int j = 0; j < kTPW; ++j)
-                            if ((wmask >> j) & 1u) or64(acc0[j], q[j * 64 + k]);
+                        for (uint32_t u = 0; u < kAtOnce; ++u) {
+                            const int ka = __ffsll((long long)xa) - 1, kb = __ffsll((long long)xb) - 1;
+                            xa &= xa - 1;
+                            xb &= xb - 1;
+#pragma unroll
+                            for (int j = 0; j < kTPW; ++j) {
+                                const bool on = (wmask >> j) & 1u;
+                                va[u][j] = vb[u][j] = make_uint2(0, 0);
+                                if (on && ka >= 0) va[u][j] = *reinterpret_cast<const uint2 *>(q + j * 64 + ka);
+                                if (on && kb >= 0) vb[u][j] = *reinterpret_cast<const uint2 *>(q + j * 64 + kb);
+                            }
+                        }
+#pragma unroll
+                        for (uint32_t u = 0; u < kAtOnce; ++u)
+#pragma unroll
+                            for (int j = 0; j < kTPW; ++j) {
+                                acc0[j].x |= va[u][j].x;
+                                acc0[j].y |= va[u][j].y;
+                                acc1[j].x |= vb[u][j].x;
+                                acc1[j].y |= vb[u][j].y;
+                            }
                     }
-                    if (xb) {
-                        const int k = __ffsll((long long)xb) - 1;
-                        xb &= xb - 1;
+                    const unsigned ra = __ballot_sync(kFull, xa != 0), rb = __ballot_sync(kFull, xb != 0);
+                    if (!(ra | rb)) break;
+                    const uint32_t most = __reduce_max_sync(kFull, (uint32_t)max(__popcll(xa), __popcll(xb)));
+                    if ((uint32_t)(__popc(ra) + __popc(rb)) * kHelpRows < most) {
 #pragma unroll
-                        for (int j = 0; j < kTPW; ++j)
-                            if ((wmask >> j) & 1u) or64(acc1[j], q[j * 64 + k]);
-                    }
-                }
+                        for (int half = 0; half < 2; ++half) {
+                            unsigned left = half ? rb : ra;
+                            while (left) {
+                                const int src = __ffs(left) - 1;
+                                left &= left - 1;
+                                const uint64_t x = __shfl_sync(kFull, half ? xb : xa, src);
+                                const uint32_t m0 = bitmask((uint32_t)x, (int)lane), m1 = bitmask((uint32_t)(x >> 32), (int)lane);
 #pragma unroll
-                for (int half = 0; half < 2; ++half) {
-                    uint64_t &xr = half ? xb : xa;
-                    unsigned left = __ballot_sync(kFull, xr != 0);
-                    while (left) {
-                        const int src = __ffs(left) - 1;
-                        left &= left - 1;
-                        const uint64_t x = __shfl_sync(kFull, xr, src);
-                        const uint32_t lo = (uint32_t)x, hi = (uint32_t)(x >> 32), nlo = __popc(lo);
-                        const uint32_t cnt = nlo + __popc(hi);
-                        uint64_t o[kTPW];
-#pragma unroll
-                        for (int j = 0; j < kTPW; ++j) o[j] = 0;
-                        for (uint32_t b = lane; b < cnt; b += 32) {
-                            const uint32_t k = b < nlo ? nth_bit(lo, b) : 32 + nth_bit(hi, b - nlo);
-#pragma unroll
-                            for (int j = 0; j < kTPW; ++j)
-                                if ((wmask >> j) & 1u) o[j] |= q[j * 64 + k];
+                                for (int j = 0; j < kTPW; ++j) {
+                                    if (!((wmask >> j) & 1u)) continue;
+                                    const uint2 q0 = *reinterpret_cast<const uint2 *>(q + j * 64 + lane);
+                                    const uint2 q1 = *reinterpret_cast<const uint2 *>(q + j * 64 + 32 + lane);
+                                    const uint32_t ox = __reduce_or_sync(kFull, (q0.x & m0) | (q1.x & m1));
+                                    const uint32_t oy = __reduce_or_sync(kFull, (q0.y & m0) | (q1.y & m1));
+                                    if ((int)lane == src) {
+                                        uint2 &acc = half ? acc1[j] : acc0[j];
+                                        acc.x |= ox;
+                                        acc.y |= oy;
+                                    }
+                                }
+                            }
                         }
-#pragma unroll
-                        for (int j = 0; j < kTPW; ++j) {
-                            if (!((wmask >> j) & 1u)) continue;
-#pragma unroll
-                            for (int d = 16; d > 0; d >>= 1) o[j] |= __shfl_xor_sync(kFull, o[j], d);
-                        }
-                        if ((int)lane == src) {
-#pragma unroll
-                            for (int j = 0; j < kTPW; ++j) or64(half ? acc1[j] : acc0[j], o[j]);
-                        }
+                        break;
                     }
                 }
             }
