@@ -476,7 +476,8 @@ typedef struct cfpq_selector_config {
     float range_margin;     /* MLP: features within the training range widened by this fraction */
     uint32_t min_tiles;     /* a single-query closure selects only if it has a term of
                                n >= 64 * min_tiles (smaller ones are latency-bound and run
-                               LOP3 throughout); batches of queries always select */
+                               LOP3 until an iteration is heavy, then select);
+                               batches of queries always select */
 } cfpq_selector_config;
 int cfpq_selector_configure(cfpq_ctx *ctx, const cfpq_selector_config *cfg);
 int cfpq_selector_get_config(cfpq_ctx *ctx, cfpq_selector_config *cfg);
