@@ -13,7 +13,7 @@
 // 4-bit operands are K-major on both sides, so one of them has to be transposed
 // bit by bit.  The block is computed as C^T = Q^T P^T: M is 128 columns of Q (2
 // tiles), N is 256 rows of P (4 tiles), and it is the smaller side that is
-// transposed, in registers (transpose_rows, 5 shuffles per 64 x 32 bits).  Work
+// transposed, in registers (Transposer, 5 shuffles per 64 x 32 bits).  Work
 // item (item list 2) = (product, group of 4 output tile-rows, block of 4 output
 // tiles), done as two halves of 2 tile columns over the whole inner dimension.
 //
@@ -24,7 +24,7 @@
 //   A warps    2 groups x 8: 32 columns of Q for half of a stage's k-tiles,
 //              transposed and expanded to TENSOR MEMORY (tcgen05.st), from where
 //              the MMA takes A;
-//   B warps    2 groups x 4: one tile row of P each, expanded to shared memory
+//   B warps    2 groups x 4: one of the 4 P tiles each, expanded to shared memory
 //              (no-swizzle K-major: 8-row x 16-byte core matrices);
 //              group g takes the operand stages of parity g (kKt k-tiles each),
 //              with the packed words loaded from global memory (L2) one unit of
