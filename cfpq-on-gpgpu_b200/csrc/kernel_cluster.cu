@@ -17,8 +17,10 @@
 // (R = 16, 32 or 64 rows: n <= 256, 512, 1024), row-major, T words a row, three
 // copies: the current matrix and two deltas used alternately.  A delta row counts
 // only while its bit is set in the delta's row mask; every CTA holds the masks
-// of all rows (whoever finds new bits sets the row's bit in all 16 copies), so
-// empty rows are never read and nothing is cleared between iterations.
+// of all rows (whoever finds new bits sets the row's bit in all 16 copies of the
+// delta's mask, and each CTA adds those to its own copy of the matrix's:
+// cluster_rows.cuh), so empty rows are never read and nothing is cleared between
+// iterations.
 //
 // Iteration t: the rules with a non-empty delta are picked, and a warp takes 32 /
 // kTp rows r of a head C, kTp lanes a row, a word per lane.  For every picked
@@ -34,7 +36,10 @@
 // tiles): when the next iteration would read more than leave_reads rows per
 // CTA, the cluster writes matrices and deltas back and leaves; the persistent
 // kernel goes on from there.  Everything a barrier waits for is decided from
-// counts that all CTAs hold alike, so all of them leave in the same iteration.
+// counts and masks that all CTAs hold alike between two barriers, also while one
+// of them is an iteration ahead (cluster_rows.cuh), so all of them leave in the
+// same iteration.
+#include "cluster_rows.cuh"
 #include "launch.h"
 
 namespace cfpq {
@@ -109,33 +114,26 @@ __global__ void __launch_bounds__(kThreads, 1) k_closure_cluster(const __grid_co
     const uint32_t group = lane / kTp, sub = lane % kTp;
     const uint32_t nm = a.nm, T = a.T, log2r = a.log2r, R = 1u << log2r, n = a.n;
     const uint32_t mat = T << log2r;  // words of one matrix's rows
-    uint64_t *const cur = sm, *const dlt = sm + (size_t)nm * mat, *const dmask = dlt + 2 * (size_t)nm * mat,
-                    *const cmask = dmask + 3 * nm * T;
-    uint16_t *const lists = reinterpret_cast<uint16_t *>(cmask + nm * T) + warp * kList, *const list = lists + group * kCap;
-    uint32_t *const cnt = reinterpret_cast<uint32_t *>(cmask + nm * T + kWarps * kList / 4);  // [3][32]
+    uint64_t *const cur = sm, *const dlt = sm + (size_t)nm * mat, *const masks = dlt + 2 * (size_t)nm * mat,
+                    *const behind = masks + 4 * nm * T;
+    uint16_t *const lists = reinterpret_cast<uint16_t *>(behind) + warp * kList, *const list = lists + group * kCap;
+    uint32_t *const cnt = reinterpret_cast<uint32_t *>(behind + kWarps * kList / 4);  // [3][32]
+    const ClusterRows rows{masks, masks + 3 * nm * T, cnt, nm, T};
     uint32_t *const newrow = cnt + 96;   // [32][2]: rows of this CTA with new bits, per head
     uint32_t *const newbits = newrow + 64;  // [32]
     const uint32_t row0 = rank << log2r, mine = row0 < n ? min(R, n - row0) : 0u;
 
-    for (uint32_t i = tid; i < 4 * nm * T; i += kThreads) dmask[i] = 0;  // and cmask behind them
-    if (tid < 192) cnt[tid] = 0;                                         // and newrow, newbits
+    for (uint32_t i = tid; i < 4 * nm * T; i += kThreads) masks[i] = 0;
+    if (tid < 192) cnt[tid] = 0;  // and newrow, newbits
     cluster_barrier();  // every CTA's masks and counts are zero before anyone adds to them
 
     // rows of matrix m with new bits (two words of row bits, this CTA's rows)
     // and their number, into every CTA's masks and counts (one warp)
     auto publish = [&](uint32_t m, uint32_t buf, uint32_t lo, uint32_t hi, uint32_t add) {
         if (lane >= kCtas) return;
-        const uint32_t d = map_rank(smem_addr(dmask + (buf * nm + m) * T + (row0 >> 6)), lane);
-        const uint32_t c = map_rank(smem_addr(cmask + m * T + (row0 >> 6)), lane);
-        if (lo) {
-            red_or_cluster(d, lo);
-            red_or_cluster(c, lo);
-        }
-        if (hi) {
-            red_or_cluster(d + 4, hi);
-            red_or_cluster(c + 4, hi);
-        }
-        red_add_cluster(map_rank(smem_addr(cnt + buf * 32 + m), lane), add);
+        rows.publish(buf, m, row0 >> 6, lo, hi, add,
+                     [&](uint32_t *p, uint32_t v) { red_or_cluster(map_rank(smem_addr(p), lane), v); },
+                     [&](uint32_t *p, uint32_t v) { red_add_cluster(map_rank(smem_addr(p), lane), v); });
     };
     // (one lane) rows `bits` (from row r on) of slot i have `add` new bits
     auto note = [&](uint32_t i, uint32_t r, uint32_t bits, uint32_t add) {
@@ -194,14 +192,13 @@ __global__ void __launch_bounds__(kThreads, 1) k_closure_cluster(const __grid_co
     unsigned long long done_ns = 0;
     bool left = false, changed = false;
     for (;; ++t) {
-        const uint32_t it = t - t0, rd = it % 3, wr = (it + 1) % 3, par = it & 1;
+        const uint32_t it = t - t0, rd = ClusterRows::read_buffer(it), wr = ClusterRows::write_buffer(it), par = it & 1;
         if (rank == 0 && tid == 0 && a.phase_log && it < a.phase_log_iters)
             a.phase_log[3 * it] = globaltimer_ns();
-        for (uint32_t i = tid; i < nm * T; i += kThreads) dmask[((it + 2) % 3) * nm * T + i] = 0;
-        if (tid < 32) cnt[((it + 2) % 3) * 32 + tid] = 0;
+        rows.open(it, tid, kThreads);
         const uint64_t *const D = dlt + par * (size_t)nm * mat;
         uint64_t *const Dn = dlt + (par ^ 1) * (size_t)nm * mat;
-        const uint64_t *const dm = dmask + rd * nm * T;
+        const uint64_t *const dm = rows.delta_rows(rd, 0);
         // the terms with a non-empty delta (iteration 0: A * B once, as the first
         // term), and the heads that have one
         uint64_t on0 = 0, on1 = 0;
@@ -284,7 +281,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_closure_cluster(const __grid_co
                 if ((on0 >> ru) & 1u) {
                     const bool fresh = valid && (it == 0 || ((dm[b1 * T + (row >> 6)] >> (row & 63)) & 1u));
                     const uint64_t *const P = it == 0 ? cur : D;
-                    gather(fresh ? P[((b1 << log2r) + r) * T + w] & cmask[b2 * T + w] : 0ULL, cur + (size_t)b2 * mat);
+                    gather(fresh ? P[((b1 << log2r) + r) * T + w] & rows.rows(rd, b2, w) : 0ULL, cur + (size_t)b2 * mat);
                 }
                 if ((on1 >> ru) & 1u)
                     gather(valid ? cur[((b1 << log2r) + r) * T + w] & dm[b2 * T + w] : 0ULL, D + (size_t)b2 * mat);
@@ -336,18 +333,18 @@ __global__ void __launch_bounds__(kThreads, 1) k_closure_cluster(const __grid_co
             if (h * 32 + lane < a.rules.nrules) est += f1 + (f2 ? n1 : 0u);
         }
         if (__reduce_add_sync(kFull, est) > limit) {
-            uint32_t rows = 0, drows = 0;  // non-empty rows of matrix `lane` and of its delta
+            uint32_t nrows = 0, ndelta = 0;  // non-empty rows of matrix `lane` and of its delta
             if (lane < nm)
                 for (uint32_t w = 0; w < T; ++w) {
-                    rows += __popcll(cmask[lane * T + w]);
-                    drows += __popcll(dmask[(wr * nm + lane) * T + w]);
+                    nrows += __popcll(rows.rows(wr, lane, w));
+                    ndelta += __popcll(rows.delta_rows(wr, lane)[w]);
                 }
             est = 0;
 #pragma unroll
             for (uint32_t h = 0; h < 2; ++h) {
                 if (h >= halves) break;
                 const uint32_t f1 = __shfl_sync(kFull, fresh, b1s[h]), n1 = __shfl_sync(kFull, total, b1s[h]);
-                const uint32_t r2 = __shfl_sync(kFull, rows, b2s[h]), d2 = __shfl_sync(kFull, drows, b2s[h]);
+                const uint32_t r2 = __shfl_sync(kFull, nrows, b2s[h]), d2 = __shfl_sync(kFull, ndelta, b2s[h]);
                 if (h * 32 + lane < a.rules.nrules)
                     est += (uint32_t)(((float)f1 * (float)r2 + (float)n1 * (float)d2) / (float)n);
             }
@@ -357,7 +354,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_closure_cluster(const __grid_co
     }
 
     // ---- write back what changed (and, on leaving, the deltas) ----
-    const uint32_t wr = (t - t0 + 1) % 3, par = (t - t0) & 1;
+    const uint32_t wr = ClusterRows::write_buffer(t - t0), par = (t - t0) & 1;
     auto put = [&](const DevMat &m, const uint64_t *src, uint32_t r, uint32_t w, bool valid) {
         const uint32_t row = row0 + r, ti = row0 >> 6;  // R divides 64: the CTA's rows lie in one tile-row
         uint32_t add = 0;
@@ -383,7 +380,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_closure_cluster(const __grid_co
         put(a.slots[head].cur, cur + (size_t)head * mat, r, w, in && r < mine);
         if (left) {
             const uint32_t row = row0 + r;
-            const bool fresh = in && r < mine && ((dmask[(wr * nm + head) * T + (row >> 6)] >> (row & 63)) & 1u);
+            const bool fresh = in && r < mine && ((rows.delta_rows(wr, head)[row >> 6] >> (row & 63)) & 1u);
             put(a.slots[head].dlt[(t + 1) & 1], dlt + ((par ^ 1) * (size_t)nm + head) * mat, r, w, fresh);
         }
     }
