@@ -1748,7 +1748,8 @@ static ClusterRules cluster_rules(const QueryIn &q) {
 // iterations became heavy: the persistent kernel has left after iteration
 // st->iter - 1 with the deltas ready for the next one; the counters are
 // measured and the multi-kernel loop with selection runs
-// to the fixpoint (result lines wanted are hashed again).
+// to the fixpoint (result lines wanted are hashed again).  The caller
+// synchronises.
 static int finish_selected(cfpq_ctx *ctx, ClosurePlan &pl, const QueryTrack &qt, uint32_t nslots, const HashOut *ho) {
     struct Stage {  // the plan's selecting view, put back on every way out
         cfpq_ctx *ctx;
@@ -1773,7 +1774,6 @@ static int finish_selected(cfpq_ctx *ctx, ClosurePlan &pl, const QueryTrack &qt,
     CUDA_TRY(cudaEventRecord(ctx->ev1, ctx->stream));
     CUDA_TRY(cudaMemcpyAsync(ctx->h_st, ctx->d_st, sizeof(IterState), cudaMemcpyDeviceToHost, ctx->stream));
     if (ho && ho->n) TRY(enqueue_hash_many(ctx, ho->mats, ho->n));
-    CUDA_TRY(cudaStreamSynchronize(ctx->stream));
     return CFPQ_OK;
 }
 
@@ -2019,9 +2019,15 @@ static int run_engine(cfpq_ctx *ctx, const std::vector<QueryIn> &qs, const cfpq_
         }
         h_done = static_cast<unsigned long long *>(ctx->h_query);
         h_last = reinterpret_cast<uint32_t *>(h_done + nq);
+    }
+    // after every stage of the closure: the ones behind it change them
+    auto read_queries = [&]() -> int {
+        if (!want_q) return CFPQ_OK;
         CUDA_TRY(cudaMemcpyAsync(h_done, qt.done_ns, nq * 8, cudaMemcpyDeviceToHost, ctx->stream));
         CUDA_TRY(cudaMemcpyAsync(h_last, qt.last_iter, nq * 4, cudaMemcpyDeviceToHost, ctx->stream));
-    }
+        return CFPQ_OK;
+    };
+    TRY(read_queries());
     // (a closure that left its kernel before the fixpoint is hashed when it is done)
     if (ho && ho->n) TRY(enqueue_hash_many(ctx, ho->mats, ho->n, pl.late_select ? &ctx->d_st->active : nullptr));
     if (ho && ho->flag_src && !flag_mapped)
@@ -2035,13 +2041,18 @@ static int run_engine(cfpq_ctx *ctx, const std::vector<QueryIn> &qs, const cfpq_
         CUDA_TRY(cudaEventRecord(ctx->ev1, ctx->stream));
         if (!st_mapped)
             CUDA_TRY(cudaMemcpyAsync(ctx->h_st, ctx->d_st, sizeof(IterState), cudaMemcpyDeviceToHost, ctx->stream));
+        TRY(read_queries());
         if (ho && ho->n) TRY(enqueue_hash_many(ctx, ho->mats, ho->n, &ctx->d_st->active));
         CUDA_TRY(cudaStreamSynchronize(ctx->stream));
     }
     ctx->phase_log_iters = persistent ? std::min<uint32_t>(hs.iter - (moved ? cluster_iters : 0), kPhaseLogIters) : 0;
     const uint32_t persistent_iters = persistent ? hs.iter : 0;
     const bool left = persistent && hs.left && !hs.error;
-    if (left) TRY(finish_selected(ctx, pl, qt, nslots, ho));
+    if (left) {
+        TRY(finish_selected(ctx, pl, qt, nslots, ho));
+        TRY(read_queries());
+        CUDA_TRY(cudaStreamSynchronize(ctx->stream));
+    }
     float ms = 0;
     CUDA_TRY(cudaEventElapsedTime(&ms, ctx->ev0, ctx->ev1));
     const bool converged = hs.last_changed == 0;
