@@ -11,7 +11,7 @@ void selector_defaults(SelectorParams *sp) {
     sp->mode = CFPQ_SELECT_HEURISTIC;
     sp->allowed = (1u << CFPQ_VARIANT_LOP3) | (1u << CFPQ_VARIANT_M4R) | (1u << CFPQ_VARIANT_TC);
     // Until cfpq_autotune runs: tensor cores for n >= 768 when a tenth of the P
-    // tiles are occupied and 10% of them dense (dense_tile_pop).  Measured on
+    // tiles are occupied and 10% of them count (tc_tile_pop).  Measured on
     // whole closures, whose tensor-core terms share one plan and one product
     // launch per iteration: sizes from 16, 12 and 8 tiles on give 13.2, 12.4 and
     // 12.2 ms for 40 mixed queries, 1225, 1247 and 1233 us for a random CNF at n =

@@ -109,25 +109,37 @@ struct MatRows {
 // Statistics of one buffer of a closure (a slot's current matrix or one of
 // its two deltas), kept exact by the product epilogues and reset when a delta
 // is cleared: population, occupied tiles (occupancy bits), dense tiles
-// (population > dense_tile_pop(T)).  Buffer b of slot s is counters[3*s + b]
-// (b = 0: current matrix, 1 + d: delta d).  They are the selector's features.
+// (population > kDenseTilePop: the selector's features and Four Russians rule),
+// tiles that count for the tensor cores (population > tc_tile_pop(T)).  Buffer b
+// of slot s is counters[3*s + b] (b = 0: current matrix, 1 + d: delta d).
 struct BufCounters {
     unsigned long long nnz;
     uint32_t occ_tiles;
     uint32_t dense_tiles;
+    uint32_t tc_tiles;
+    uint32_t pad;
 };
-// A tile counts as dense from the population on at which the cheaper of the
-// word-level kernels loses to the variant that would take its product.  Sizes
-// that the tensor cores take (kTcTiles..2048 tiles): more than kTcTilePop bits.
-// A k-tile costs them the same whatever it holds; by itself a product at n =
-// 8192 breaks even at 8 bits a tile (257 against 242 us; 257 against 560 at 82),
-// and in a closure, whose tiles fill up within an iteration, earlier: limits of
-// 96, 40, 16, 8 and 4 bits give 313, 287, 262, 253 and 230 ms for the chain closure
-// at n = 16384, 3.37, 3.21, 2.40, 2.42 and 2.12 ms for a random CNF at n = 3001.
-// Elsewhere Four Russians are the alternative, ahead only above kDenseTilePop
-// (560 us for LOP3 against 800 at 82 bits, 1400 against 935 at 1200).
+// Two limits of a tile's population, since the alternatives to LOP3 pass it at
+// different ones.  Single products with random bits, us by LOP3 / Four Russians /
+// tensor cores:
+//   bits a tile        4           8          16          82         205         410         819
+//   n = 8192  193/293/258 210/316/257 245/352/258 382/538/259 579/774/257 850/932/259 1409/933/258
+//   n = 5003    70/96/91   75/104/90   82/117/91  118/158/90  169/210/90  235/249/90   359/295/91
+// kDenseTilePop, for the Four Russians rule and the features: closures fill their
+// tiles within an iteration, so the limit matters less there than for a single
+// product, which breaks even between 410 and 819 bits.  With the tensor cores
+// excluded, limits of 96, 256 and 512 bits give 1078, 1089 and 1117 ms for the
+// chain closure at n = 16384, 3.98, 3.93 and 4.12 ms for a random CNF at n = 3001.
+// tc_tile_pop(T), for the tensor-core rule and the merging of a rule's terms: sizes
+// that the tensor cores take (kTcTiles..2048 tiles) count tiles of more than
+// kTcTilePop bits.  A k-tile costs them the same whatever it holds; by itself a
+// product breaks even at 16 to 32 bits a tile, in a closure earlier: limits of 96,
+// 40, 16, 8 and 4 bits gave 313, 287, 262, 253 and 230 ms for the chain closure at
+// n = 16384, 3.37, 3.21, 2.40, 2.42 and 2.12 ms for a random CNF at n = 3001.  One
+// limit of 4 bits for both rules sent light tiles to Four Russians where the
+// tensor cores did not take them: that chain 222 ms, now 214.
 constexpr uint32_t kDenseTilePop = 96, kTcTilePop = 4, kTcTiles = 12;
-__host__ __device__ constexpr uint32_t dense_tile_pop(uint32_t T) {
+__host__ __device__ constexpr uint32_t tc_tile_pop(uint32_t T) {
     return T >= kTcTiles && T <= 2048 ? kTcTilePop : kDenseTilePop;
 }
 
@@ -365,16 +377,17 @@ __device__ __forceinline__ void tiles_gain(const DevMat &m, uint32_t ti, uint32_
                                            BufCounters *cnt) {
     const uint32_t lane = threadIdx.x & 31;
     const uint32_t tj = tj0 + lane;
-    uint32_t gained = 0, dense = 0;
-    const uint32_t limit = dense_tile_pop(m.T);
+    uint32_t gained = 0;  // occupied, dense and tensor-core tiles gained, 8 bits each
     if (lane < 4 && add) {
         const size_t t = (size_t)ti * m.T + tj;
         const uint32_t bit = 1u << (tj & 31);
         if (cnt) {
             const uint32_t old_pop = atomicAdd(m.nnz + t, add);
             const uint32_t old_occ = atomicOr(m.occ + (size_t)ti * m.ow + (tj >> 5), bit);
+            const uint32_t limit = tc_tile_pop(m.T);
             gained = (old_occ & bit) ? 0u : 1u;
-            dense = (old_pop <= limit && old_pop + add > limit) ? 1u : 0u;
+            if (old_pop <= kDenseTilePop && old_pop + add > kDenseTilePop) gained |= 1u << 8;
+            if (old_pop <= limit && old_pop + add > limit) gained |= 1u << 16;
         } else {
             atomicAdd(m.nnz + t, add);
             atomicOr(m.occ + (size_t)ti * m.ow + (tj >> 5), bit);
@@ -383,11 +396,11 @@ __device__ __forceinline__ void tiles_gain(const DevMat &m, uint32_t ti, uint32_
     if (!cnt) return;
     const uint32_t sum_add = __reduce_add_sync(0xffffffffu, lane < 4 ? add : 0u);
     const uint32_t sum_gained = __reduce_add_sync(0xffffffffu, gained);
-    const uint32_t sum_dense = __reduce_add_sync(0xffffffffu, dense);
     if (lane == 0) {
         if (sum_add) atomicAdd(&cnt->nnz, sum_add);
-        if (sum_gained) atomicAdd(&cnt->occ_tiles, sum_gained);
-        if (sum_dense) atomicAdd(&cnt->dense_tiles, sum_dense);
+        if (sum_gained & 0xffu) atomicAdd(&cnt->occ_tiles, sum_gained & 0xffu);
+        if ((sum_gained >> 8) & 0xffu) atomicAdd(&cnt->dense_tiles, (sum_gained >> 8) & 0xffu);
+        if (sum_gained >> 16) atomicAdd(&cnt->tc_tiles, sum_gained >> 16);
     }
 }
 

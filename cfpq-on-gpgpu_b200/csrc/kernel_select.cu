@@ -21,7 +21,7 @@
 //   0 log2 n / 17            1 term (0: dA*B, 1: A*dB)
 //   2 P occupied-tile frac   3 Q occupied-tile frac
 //   4 P mean tile population / 4096          5 same for Q
-//   6 P dense-tile fraction (population > dense_tile_pop(T)) of occupied   7 same for Q
+//   6 P dense-tile fraction (population > kDenseTilePop) of occupied   7 same for Q
 //   8 log2(1 + nnz P) / 34   9 log2(1 + nnz Q) / 34
 //  10 nnz of the delta operand / nnz of its slot's current matrix
 //  11 log2(1 + occP * occQ / T) / 32  (expected tile triples, uniform tiles)
@@ -68,49 +68,53 @@ __global__ void k_counters_init(const MatSlot *__restrict__ slots, BufCounters *
     const uint32_t buf = blockIdx.y;
     const DevMat m = buf ? slots[blockIdx.x].dlt[buf - 1] : slots[blockIdx.x].cur;
     unsigned long long nnz = 0;
-    uint32_t occ = 0, dense = 0;
+    uint32_t occ = 0, dense = 0, tc = 0;
     const size_t tiles = (size_t)m.T * m.T, words = (size_t)m.T * m.ow;
-    const uint32_t limit = dense_tile_pop(m.T);
+    const uint32_t limit = tc_tile_pop(m.T);
     for (size_t i = threadIdx.x; i < tiles; i += blockDim.x) {
         const uint32_t pop = m.nnz[i];
         nnz += pop;
-        dense += pop > limit;
+        dense += pop > kDenseTilePop;
+        tc += pop > limit;
     }
     for (size_t i = threadIdx.x; i < words; i += blockDim.x) occ += __popc(m.occ[i]);
     __shared__ unsigned long long s_nnz[32];
-    __shared__ uint32_t s_occ[32], s_dense[32];
+    __shared__ uint32_t s_occ[32], s_dense[32], s_tc[32];
     for (int d = 16; d > 0; d >>= 1) {
         nnz += __shfl_xor_sync(kFull, nnz, d);
         occ += __shfl_xor_sync(kFull, occ, d);
         dense += __shfl_xor_sync(kFull, dense, d);
+        tc += __shfl_xor_sync(kFull, tc, d);
     }
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
     if (lane == 0) {
         s_nnz[warp] = nnz;
         s_occ[warp] = occ;
         s_dense[warp] = dense;
+        s_tc[warp] = tc;
     }
     __syncthreads();
     if (threadIdx.x == 0) {
-        BufCounters c = {0, 0, 0};
+        BufCounters c{};
         for (uint32_t w = 0; w < nw; ++w) {
             c.nnz += s_nnz[w];
             c.occ_tiles += s_occ[w];
             c.dense_tiles += s_dense[w];
+            c.tc_tiles += s_tc[w];
         }
         cnts[3 * blockIdx.x + buf] = c;
         if (gridDim.y == 1) {
-            cnts[3 * blockIdx.x + 1] = BufCounters{0, 0, 0};
-            cnts[3 * blockIdx.x + 2] = BufCounters{0, 0, 0};
+            cnts[3 * blockIdx.x + 1] = BufCounters{};
+            cnts[3 * blockIdx.x + 2] = BufCounters{};
         }
     }
 }
 
 // Variant of one product by itself (cfpq_add_mul with AUTO): the heuristic's
 // tensor-core rule on the left operand's tile statistics, with tiles of more
-// than 16 bits as the dense ones: the operands do not fill up as in a closure,
-// and at n = 8192 LOP3 takes 242 us at 8 bits a tile and 560 at 82, the tensor
-// cores 257.  One block.
+// than 16 bits as the ones that count: the operands do not fill up as in a closure,
+// and the break-even lies there (n = 8192: LOP3 takes 245 us at 16 bits a tile and
+// 275 at 32, the tensor cores 258; n = 5003: 82 and 91 against 91).  One block.
 constexpr uint32_t kAddMulTilePop = 16;
 __global__ void __launch_bounds__(1024) k_add_mul_choose(DevMat a, float min_occ, float min_dense, uint32_t *use_tc) {
     const uint32_t tiles = a.T * a.T, words = a.T * a.ow;

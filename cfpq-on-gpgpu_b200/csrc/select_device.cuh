@@ -36,7 +36,7 @@ __device__ __forceinline__ bool merge_terms(const ProdDesc &pd, const BufCounter
     const float occA = static_counts ? fmaxf((float)cnts[3 * pd.pslot].occ_tiles, 1.f) : T2;
     const float occB = static_counts ? fmaxf((float)cnts[3 * pd.qslot].occ_tiles, 1.f) : T2;
     const float a = fminf((float)DA.occ_tiles / occA, 1.f), b = fminf((float)DB.occ_tiles / occB, 1.f);
-    const float dense = (float)DA.dense_tiles / (float)DA.occ_tiles;
+    const float dense = (float)DA.tc_tiles / (float)DA.occ_tiles;
     return a * (0.3f + 0.7f * dense) + b > 1.1f * (a + b - a * b);
 }
 
@@ -70,13 +70,16 @@ __device__ __forceinline__ void product_features(const ProdDesc &pd, const BufCo
     f[15] = 0.f;
 }
 
-__device__ __forceinline__ uint32_t heuristic_choice(const SelectorParams &sp, const float *f, uint32_t T, bool tc_ok) {
+// tc_share: share of P's occupied tiles that count for the tensor cores.
+__device__ __forceinline__ uint32_t heuristic_choice(const SelectorParams &sp, const float *f, float tc_share,
+                                                     uint32_t T, bool tc_ok) {
     const uint32_t allowed = sp.allowed;
     // tensor cores: a k-tile costs them the same whatever the tiles hold, so
     // they win where the word-level kernels pay full tiles too -- dense P
     // tiles, whose cost does not depend on Q's population or occupancy --
     // and the product is not tiny
-    if (tc_ok && (allowed & (1u << 4)) && T >= sp.tc_min_tiles && f[2] >= sp.tc_min_occ && f[6] >= sp.tc_min_dense)
+    if (tc_ok && (allowed & (1u << 4)) && T >= sp.tc_min_tiles && f[2] >= sp.tc_min_occ &&
+        tc_share >= sp.tc_min_dense)
         return 4;
     if ((allowed & (1u << 3)) && f[6] >= sp.m4r_min_dense) return 3;
     if (allowed & (1u << 2)) return 2;
@@ -124,7 +127,8 @@ __device__ __forceinline__ uint32_t select_product(const ProdDesc &pd, const Buf
                                                    const SelectorParams *sp, bool tcp, float *f, float *pred,
                                                    uint32_t *flags_out) {
     product_features(pd, cnts, iter, f);
-    uint32_t v = heuristic_choice(*sp, f, pd.T, tcp);
+    const BufCounters P = cnts[operand_buffer(pd.pslot, pd.p_delta, iter)];
+    uint32_t v = heuristic_choice(*sp, f, P.occ_tiles ? (float)P.tc_tiles / (float)P.occ_tiles : 0.f, pd.T, tcp);
     uint32_t flags = 0;
     if (sp->mode == 2 && sp->has_weights) {
         selector_mlp_warp(sp->w, f, pred);

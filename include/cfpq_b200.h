@@ -467,11 +467,10 @@ typedef struct cfpq_selector_config {
     uint32_t allowed;       /* bit v set: variant v may be chosen (bits 2, 3, 4) */
     uint32_t tc_min_tiles;  /* tensor cores only for n >= 64 * tc_min_tiles */
     float tc_min_occ;       /* TC: minimum occupied-tile fraction of P */
-    float tc_min_dense;     /* TC: minimum fraction of dense P tiles (population > 4 for
-                               768 <= n <= 131072, where the tensor cores are the
-                               alternative, > 96 elsewhere): the word-level kernels pay by
+    float tc_min_dense;     /* TC: minimum fraction of P tiles with a population > 4 (> 96 for
+                               n < 705 and n > 131072): the word-level kernels pay by
                                population, the tensor cores the same for every tile */
-    float m4r_min_dense;    /* M4R: minimum fraction of dense P tiles */
+    float m4r_min_dense;    /* M4R: minimum fraction of dense P tiles (population > 96) */
     float conf_margin;      /* MLP: best prediction ahead of the second by this (log us) */
     float range_margin;     /* MLP: features within the training range widened by this fraction */
     uint32_t min_tiles;     /* a single-query closure selects only if it has a term of
