@@ -6,6 +6,10 @@
 
 #include "ctx.h"
 
+// Shares of the occupied P tiles above which a rule takes its variant, and of all
+// tiles that have to be occupied (selector_defaults; the autotuner sets the same).
+constexpr float kTcMinOcc = 0.1f, kTcMinDense = 0.1f, kM4rMinDense = 0.25f;
+
 void selector_defaults(SelectorParams *sp) {
     memset(sp, 0, sizeof(*sp));
     sp->mode = CFPQ_SELECT_HEURISTIC;
@@ -20,9 +24,9 @@ void selector_defaults(SelectorParams *sp) {
     // Russians when a quarter of the P tiles are dense.  (A single query selects from n >= 64 * min_tiles,
     // and below once its iterations are heavy.)
     sp->tc_min_tiles = kTcTiles;
-    sp->tc_min_occ = 0.1f;
-    sp->tc_min_dense = 0.1f;
-    sp->m4r_min_dense = 0.25f;
+    sp->tc_min_occ = kTcMinOcc;
+    sp->tc_min_dense = kTcMinDense;
+    sp->m4r_min_dense = kM4rMinDense;
     sp->conf_margin = 0.05f;
     sp->range_margin = 0.1f;
     // Per-iteration selection costs one feature computation per planned row
@@ -354,39 +358,53 @@ extern "C" int cfpq_autotune(cfpq_ctx *ctx, const cfpq_autotune_opts *opts, cfpq
         TRY(rc);
     }
     // Crossovers.  Random inputs populate every tile with mean population
-    // density * 4096, so the density is the tile population the features see.
+    // density * 4096, so the density is the tile population that the rules count.
+    // A rule takes its variant for all tiles above its limit alike, and closures
+    // pass through all of those populations, so the times are added up over them:
+    // one density that LOP3 wins (410 bits since its sparse loop takes tiles of up
+    // to 512) says little against three that it loses by half.
     SelectorParams &sp = ctx->sel;
-    auto T = [&](size_t si, size_t di, int v) { return t[(si * o.ndensities + di) * 3 + v]; };
-    // Four Russians: chosen when it beats LOP3 on every size at every density
-    // whose tiles are dense (population above 96 bits)
-    bool m4r_wins = true, any_dense = false;
-    for (size_t si = 0; si < o.nsizes; ++si)
-        for (size_t di = 0; di < o.ndensities; ++di)
-            if (o.densities[di] * 4096.f > (float)kDenseTilePop) {
-                any_dense = true;
-                m4r_wins = m4r_wins && T(si, di, 1) > 0 && T(si, di, 1) < T(si, di, 0);
-            }
-    sp.m4r_min_dense = (any_dense && m4r_wins) ? 0.25f : 1.5f;
-    // tensor cores: the smallest size at which TC beats both word-level
-    // variants at every density whose tiles are dense sets tc_min_tiles (the
-    // rule then takes TC where most P tiles are dense); no such size: never
-    sp.tc_min_dense = 2.f;
-    bool found = false;
-    for (size_t si = 0; si < o.nsizes && ctx->tc_grid; ++si) {
-        bool wins = false;
+    auto sum = [&](size_t si, uint32_t limit, int v) {  // ms of variant v, word level (best) for v < 0; < 0: none
+        double ms = 0;
+        bool any = false;
         for (size_t di = 0; di < o.ndensities; ++di) {
-            if (o.densities[di] * 4096.f <= (float)kDenseTilePop) continue;
-            const float tc = T(si, di, 2), w = std::min(T(si, di, 0), T(si, di, 1) > 0 ? T(si, di, 1) : 1e30f);
-            wins = tc > 0 && tc < w;
-            if (!wins) break;
+            if (o.densities[di] * 4096.f <= (float)limit) continue;
+            const float *x = &t[(si * o.ndensities + di) * 3];
+            const float one = v < 0 ? std::min(x[0], x[1]) : x[v];
+            if (one <= 0) return -1.0;
+            ms += one;
+            any = true;
         }
-        if (wins && (!found || (o.sizes[si] + 63) / 64 < sp.tc_min_tiles)) {
-            sp.tc_min_tiles = std::max<uint32_t>(1, (o.sizes[si] + 63) / 64);
-            sp.tc_min_dense = 0.3f;
-            found = true;
-        }
+        return any ? ms : -1.0;
+    };
+    // Four Russians: chosen when ahead of LOP3 over the densities whose tiles are
+    // dense and all sizes together (the rule knows no size, and at n = 2048 the
+    // two are 44 and 43 us on full tiles, at n = 8192 1409 and 931)
+    double lop3 = 0, m4r = 0;
+    for (size_t si = 0; si < o.nsizes; ++si) {
+        lop3 += std::max(sum(si, kDenseTilePop, 0), 0.0);
+        m4r += std::max(sum(si, kDenseTilePop, 1), 0.0);
     }
-    sp.tc_min_occ = 0.2f;
+    sp.m4r_min_dense = m4r < lop3 ? kM4rMinDense : 1.5f;
+    // tensor cores: the smallest size at which they are ahead of the word-level
+    // variants over the densities whose tiles count for them sets tc_min_tiles;
+    // no such size: never; ahead on every size: nothing was seen of where they
+    // stop being so, the default stays (or a smaller size that was tried)
+    sp.tc_min_dense = 2.f;
+    uint32_t smallest = 0xFFFFFFFFu;
+    bool all = true;
+    for (size_t si = 0; si < o.nsizes && ctx->tc_grid; ++si) {
+        const uint32_t T = (o.sizes[si] + 63) / 64;
+        const double tc = sum(si, tc_tile_pop(T), 2);
+        const bool wins = tc > 0 && tc < sum(si, tc_tile_pop(T), -1);
+        all = all && wins;
+        if (wins) smallest = std::min(smallest, T);
+    }
+    if (smallest != 0xFFFFFFFFu) {
+        sp.tc_min_tiles = all ? std::min(smallest, kTcTiles) : smallest;
+        sp.tc_min_dense = kTcMinDense;
+    }
+    sp.tc_min_occ = kTcMinOcc;
     if (sp.mode == CFPQ_SELECT_FIXED) sp.mode = CFPQ_SELECT_HEURISTIC;
     ctx->sel_dirty = true;
     if (result) TRY(cfpq_selector_get_config(ctx, result));

@@ -518,7 +518,9 @@ int cfpq_selector_predict(cfpq_ctx *ctx, const float *x, size_t n, float *out);
 /* Autotuner: times C |= A * B with LOP3, M4R and TC on seeded random
  * matrices (every tile populated) for the given sizes and densities, finds the
  * crossovers and stores them in the context's selector thresholds (and in
- * *result).  timings (optional, [nsizes][ndensities][3] ms, < 0 = not run). */
+ * *result).  A variant is taken where it is ahead over all densities whose tiles
+ * its rule counts, together; tensor cores that are ahead on every size keep
+ * tc_min_tiles at its default.  timings (optional, [nsizes][ndensities][3] ms, < 0 = not run). */
 typedef struct cfpq_autotune_opts {
     const uint32_t *sizes;
     size_t nsizes;
