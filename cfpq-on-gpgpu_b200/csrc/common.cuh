@@ -97,6 +97,9 @@ struct IterState {
     uint32_t exit_count;              // persistent kernel: CTAs past their exit statistics
     uint32_t left;                    // persistent kernel: left before the fixpoint (kBarLeave), still active
 };
+// (8 bytes more, and so a fifth cache line, cost closures of the persistent kernel
+// 4%: balanced brackets at n = 1024 409 -> 424 us)
+static_assert(sizeof(IterState) == 512, "IterState: four lines");
 
 // A matrix and the prefix sum of tile-rows over a list of matrices (kernels
 // with one warp per (matrix, tile-row)).

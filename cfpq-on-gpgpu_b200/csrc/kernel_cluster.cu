@@ -188,6 +188,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_closure_cluster(const __grid_co
     uint32_t fresh = lane < nm ? cnt[lane] : 0u;  // new bits of matrix `lane` in the last iteration (at first: all)
     uint32_t total = fresh;                       // its set bits
     unsigned long long reads = 0, products = 0;
+    uint32_t items = 0, outw = 0, neww = 0;  // row groups done, non-zero and new words merged
     uint32_t last_iter = 0, t = t0;
     unsigned long long done_ns = 0;
     bool left = false, changed = false;
@@ -289,6 +290,9 @@ __global__ void __launch_bounds__(kThreads, 1) k_closure_cluster(const __grid_co
             const size_t at = ((size_t)(head << log2r) + r) * T + w;
             const uint64_t old = valid ? cur[at] : 0ULL, nw = valid ? acc & ~old : 0ULL;
             const uint32_t bits = group_bits(nw != 0);
+            ++items;
+            outw += valid && acc != 0;
+            neww += nw != 0;
             if (!bits) continue;
             if (nw) cur[at] = old | nw;
             if (valid && ((bits >> group) & 1u)) Dn[at] = nw;
@@ -384,13 +388,35 @@ __global__ void __launch_bounds__(kThreads, 1) k_closure_cluster(const __grid_co
             put(a.slots[head].dlt[(t + 1) & 1], dlt + ((par ^ 1) * (size_t)nm + head) * mat, r, w, fresh);
         }
     }
-    for (int o = 16; o > 0; o >>= 1) reads += __shfl_xor_sync(kFull, reads, o);
-    if (lane == 0 && reads) atomicAdd(&a.st->new_words, reads);  // rows read, turned into tile triples below
+    for (int o = 16; o > 0; o >>= 1) {
+        reads += __shfl_xor_sync(kFull, reads, o);
+        outw += __shfl_xor_sync(kFull, outw, o);
+        neww += __shfl_xor_sync(kFull, neww, o);
+    }
+    // per CTA first, in the row collectors (all zero now): an atomic of every warp
+    // on the state's words took 6 us
+    unsigned long long *const sum = reinterpret_cast<unsigned long long *>(newrow);
+    if (lane == 0 && items) {
+        atomicAdd(sum, (unsigned long long)items);
+        atomicAdd(sum + 1, reads);
+        atomicAdd(sum + 2, (unsigned long long)outw);
+        atomicAdd(sum + 3, (unsigned long long)neww);
+    }
+    __syncthreads();
+    if (tid < 5 && sum[tid ? tid - 1 : 0]) {
+        unsigned long long *const to = tid == 0   ? &a.st->items_by_variant[2]
+                                       : tid == 1 ? &a.st->items_total
+                                       : tid == 2 ? &a.st->tile_triples  // rows read until the end
+                                       : tid == 3 ? &a.st->out_words
+                                                  : &a.st->new_words;
+        atomicAdd(to, sum[tid ? tid - 1 : 0]);
+    }
     cluster_barrier();  // every CTA's counters are in, and no CTA's shared memory is read any more
     if (rank == 0 && tid == 0) {
         IterState *const st = a.st;
-        st->tile_triples += *(volatile unsigned long long *)&st->new_words * T / 4096;  // a row read is 64 T bit pairs
-        st->new_words = 0;
+        // the rows read, of 64 T bit pairs each
+        st->tile_triples = *(volatile unsigned long long *)&st->tile_triples * T / 4096;
+        st->bytes_staged += (unsigned long long)nm * n * T * 8;
         st->products += products;
         st->dense_bitops += products * (unsigned long long)n * n * n;
         st->last_changed = changed;

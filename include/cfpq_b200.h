@@ -112,13 +112,17 @@ typedef struct cfpq_closure_stats {
     uint32_t iterations;        /* ENGINE: device iterations run; WORKLIST: 0 */
     uint32_t reserved0;
     uint64_t products;          /* rule products launched (ENGINE: non-empty product terms) */
-    uint64_t tile_triples;      /* 64x64x64 bit tile products executed */
-    uint64_t work_items;        /* output blocks processed by product kernels */
+    uint64_t tile_triples;      /* 64x64x64 bit tile products executed; in the cluster kernel
+                                   (one AUTO query, n <= 1024) the rows it read, as so many
+                                   tile products of the same bit pairs */
+    uint64_t work_items;        /* output blocks processed by product kernels (cluster kernel:
+                                   groups of 2, 4 or 8 rows of a head) */
     uint64_t dense_bitops;      /* sum over products of n^3 (dense-equivalent bit-MACs) */
     double device_ms;           /* device time of the closure (CUDA events) */
     uint64_t kernel_launches;   /* kernels launched by this call */
-    uint64_t variant_items[5];  /* work items per cfpq_variant */
-    uint64_t bytes_staged;      /* operand bytes staged global -> shared by product kernels */
+    uint64_t variant_items[5];  /* work items per cfpq_variant (the cluster kernel's: LOP3) */
+    uint64_t bytes_staged;      /* operand bytes staged global -> shared by product kernels
+                                   (cluster kernel: its matrices, once) */
     uint64_t out_words;         /* non-zero 64-bit result words merged into heads */
     uint64_t new_words;         /* result words that carried new bits */
 } cfpq_closure_stats;

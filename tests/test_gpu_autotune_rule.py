@@ -40,7 +40,7 @@ def test_autotuned_selection_is_the_measured_one(pkg):
     c = pkg.capi.Context(0)
     try:
         default = c.selector_config()
-        cfg, _ = c.autotune()
+        cfg, _ = c.autotune(reps=10)
     finally:
         c.close()
     assert cfg == default
