@@ -1520,7 +1520,7 @@ extern "C" int cfpq_last_kernel_profile(cfpq_ctx *ctx, cfpq_kernel_profile *out)
 }
 
 // Build (or reuse) the CUDA graph: one while node whose body is one iteration.
-static int get_loop_graph(cfpq_ctx *ctx, const ClosurePlan &pl, const QueryTrack &qt, cudaGraphExec_t *out) {
+static std::vector<uint64_t> loop_graph_key(const cfpq_ctx *ctx, const ClosurePlan &pl, const QueryTrack &qt) {
     std::vector<uint64_t> key = {(uint64_t)(uintptr_t)ctx->prods.p,  (uint64_t)pl.prods.size(),
                                  (uint64_t)pl.prod_rows,              (uint64_t)(uintptr_t)ctx->slots.p,
                                  (uint64_t)pl.slots.size(),           (uint64_t)pl.slot_rows,
@@ -1534,6 +1534,11 @@ static int get_loop_graph(cfpq_ctx *ctx, const ClosurePlan &pl, const QueryTrack
                                  (uint64_t)ctx->sel_log_iters,        (uint64_t)pl.auto_select};
     key.push_back((uint64_t)(uintptr_t)ctx->tc_rows.p);  // the grouped tensor-core launches
     key.push_back(((uint64_t)pl.tc_rows.size() << 32) | pl.tc_groups);
+    return key;
+}
+
+static int get_loop_graph(cfpq_ctx *ctx, const ClosurePlan &pl, const QueryTrack &qt, cudaGraphExec_t *out) {
+    const std::vector<uint64_t> key = loop_graph_key(ctx, pl, qt);
     if (ctx->gcache.exec && ctx->gcache.key == key) {
         *out = ctx->gcache.exec;
         return CFPQ_OK;
@@ -1744,12 +1749,32 @@ static ClusterRules cluster_rules(const QueryIn &q) {
     return r;
 }
 
+// Iterations launched from the host until the device flag says that the closure
+// is done: it is looked at every `batch` iterations; surplus ones after the
+// fixpoint are no-ops.
+static int run_host_loop(cfpq_ctx *ctx, const ClosurePlan &pl, const QueryTrack &qt) {
+    const int batch = 4;
+    uint32_t launched = 0;
+    for (;;) {
+        for (int k = 0; k < batch; ++k) TRY(enqueue_iteration(ctx, pl, qt, 0, 0));
+        launched += batch;
+        CUDA_TRY(cudaMemcpyAsync(ctx->h_st, ctx->d_st, sizeof(IterState), cudaMemcpyDeviceToHost, ctx->stream));
+        CUDA_TRY(cudaStreamSynchronize(ctx->stream));
+        if (!ctx->h_st->active) return CFPQ_OK;
+        if (launched > (1u << 24)) return set_error(CFPQ_ERR_CUDA, "closure did not converge");
+    }
+}
+
 // Second stage of a late-selecting closure (ClosurePlan::late_select) whose
 // iterations became heavy: the persistent kernel has left after iteration
 // st->iter - 1 with the deltas ready for the next one; the counters are
 // measured and the multi-kernel loop with selection runs
 // to the fixpoint (result lines wanted are hashed again).  The caller
-// synchronises.
+// synchronises.  The loop is a graph when the context has it, or is asked for it
+// a third time running; to build it takes 310 us, as much as half such a closure
+// (dense random CNF, n = 850 and 950 by turns: 1104 us a query with a graph for
+// each call, 852 from the host), so that a shape met for the first time and shapes
+// that take turns run from the host.
 static int finish_selected(cfpq_ctx *ctx, ClosurePlan &pl, const QueryTrack &qt, uint32_t nslots, const HashOut *ho) {
     struct Stage {  // the plan's selecting view, put back on every way out
         cfpq_ctx *ctx;
@@ -1768,9 +1793,17 @@ static int finish_selected(cfpq_ctx *ctx, ClosurePlan &pl, const QueryTrack &qt,
     TRY(selector_sync(ctx));
     CUDA_TRY(cudaMemsetAsync(qt.changed, 0, 3 * sizeof(uint32_t), ctx->stream));
     CUDA_TRY(launch_counters_init(ctx->slots.as<MatSlot>(), nslots, ctx->cnts.as<BufCounters>(), true, ctx->stream));
-    cudaGraphExec_t exec = nullptr;
-    TRY(get_loop_graph(ctx, pl, qt, &exec));
-    CUDA_TRY(cudaGraphLaunch(exec, ctx->stream));
+    std::vector<uint64_t> key = loop_graph_key(ctx, pl, qt);
+    const bool have = ctx->gcache.exec && ctx->gcache.key == key;
+    ctx->loop_asked = key == ctx->loop_key ? ctx->loop_asked + 1 : 1;
+    ctx->loop_key = std::move(key);
+    if (have || ctx->loop_asked > 2) {
+        cudaGraphExec_t exec = nullptr;
+        TRY(get_loop_graph(ctx, pl, qt, &exec));
+        CUDA_TRY(cudaGraphLaunch(exec, ctx->stream));
+    } else {
+        TRY(run_host_loop(ctx, pl, qt));
+    }
     CUDA_TRY(cudaEventRecord(ctx->ev1, ctx->stream));
     CUDA_TRY(cudaMemcpyAsync(ctx->h_st, ctx->d_st, sizeof(IterState), cudaMemcpyDeviceToHost, ctx->stream));
     if (ho && ho->n) TRY(enqueue_hash_many(ctx, ho->mats, ho->n));
@@ -1985,18 +2018,7 @@ static int run_engine(cfpq_ctx *ctx, const std::vector<QueryIn> &qs, const cfpq_
     } else if (exec) {
         CUDA_TRY(cudaGraphLaunch(exec, ctx->stream));
     } else {
-        // Host loop: check the device flag every `batch` iterations; surplus
-        // iterations after convergence are no-ops.
-        const int batch = 4;
-        uint32_t launched = 0;
-        for (;;) {
-            for (int k = 0; k < batch; ++k) TRY(enqueue_iteration(ctx, pl, qt, 0, 0));
-            launched += batch;
-            CUDA_TRY(cudaMemcpyAsync(ctx->h_st, ctx->d_st, sizeof(IterState), cudaMemcpyDeviceToHost, ctx->stream));
-            CUDA_TRY(cudaStreamSynchronize(ctx->stream));
-            if (!ctx->h_st->active) break;
-            if (launched > (1u << 24)) return set_error(CFPQ_ERR_CUDA, "closure did not converge");
-        }
+        TRY(run_host_loop(ctx, pl, qt));
     }
     CUDA_TRY(cudaEventRecord(ctx->ev1, ctx->stream));
     if (!st_mapped)

@@ -131,6 +131,8 @@ struct cfpq_ctx {
     std::unordered_map<uint32_t, PowTables> pow;
     std::vector<cfpq_matrix *> pool;  // zeroed spare matrices (deltas, alias copies)
     GraphCache gcache;
+    std::vector<uint64_t> loop_key;  // loop graph that the last closure to change loops asked for
+    uint32_t loop_asked = 0;         // times running that it did
     PlanCache *pcache = nullptr;  // created by the first closure
     uint64_t plan_ids = 0;
     uint64_t tables_owner = 0;  // plan id whose slot / product tables are in `slots` / `prods`

@@ -1,0 +1,73 @@
+"""Heavy small queries go on in the multi-kernel loop: from the host at first, as a
+graph when the same one keeps coming.  Every way gives the oracle's answer, and
+queries of different shapes that take turns do not pay for a graph in each call."""
+import time
+
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def _dense(pkg, n):
+    labels = [f"l{i}" for i in range(4)]
+    w = pkg.workloads
+    return w.Workload("dense", w.random_cnf(8, 20, labels, 4), w.uniform_graph(n, 4 * n, labels, n), {})
+
+
+def _expected(oracle, wl, tmp_path):
+    gp, rp = str(tmp_path / "g.txt"), str(tmp_path / "r.txt")
+    wl.write(gp, rp)
+    with oracle.Problem(gp, rp) as p:
+        p.closure(oracle.NAIVE, 1)
+        return p.results()
+
+
+def _call(ctx, q, wl):
+    g = wl.graph
+    st, lines = ctx.intersection(wl.grammar.rules, q.mats, g.src, g.label, g.dst, q.off, q.lm, wl.grammar.epsilon)
+    return st, dict(zip(wl.grammar.nonterminals, lines))
+
+
+def test_host_loop_and_graph_give_the_same_answers(pkg, oracle, tmp_path):
+    wls = [_dense(pkg, n) for n in (1030, 1089, 900)]
+    exp = [_expected(oracle, wl, tmp_path) for wl in wls]
+    ctx = pkg.capi.Context(0)
+    qs = [pkg.query.PreparedQuery(ctx, wl.grammar, wl.graph) for wl in wls]
+    try:
+        for i in (0, 0, 0, 0, 1, 0, 1, 2, 2, 2, 1, 1, 1, 0):
+            st, lines = _call(ctx, qs[i], wls[i])
+            assert lines == exp[i]
+            assert st["variant_items"][4] > 0  # it reached the loop that selects
+        for limit in (3, 5):  # a limit inside the loop
+            qs[1].load()
+            assert ctx.closure(wls[1].grammar.rules, qs[1].mats, max_iterations=limit)["iterations"] == limit
+            ctx.closure(wls[1].grammar.rules, qs[1].mats)
+            assert dict(zip(wls[1].grammar.nonterminals, ctx.hash_count_many(qs[1].mats))) == exp[1]
+    finally:
+        for q in qs:
+            q.close()
+        ctx.close()
+
+
+def test_turns_cost_no_graph(pkg):
+    """A graph takes 310 us to build, each of these queries 500 to 900; by turns they may take 20% more than by
+    themselves (40% with a graph in every call)."""
+    ctx = pkg.capi.Context(0)
+    wls = [_dense(pkg, n) for n in (1030, 1100)]
+    qs = [pkg.query.PreparedQuery(ctx, wl.grammar, wl.graph) for wl in wls]
+    try:
+        def best(order, reps=20):
+            times = []
+            for _ in range(reps):
+                t0 = time.perf_counter()
+                for i in order:
+                    _call(ctx, qs[i], wls[i])
+                times.append(time.perf_counter() - t0)
+            return min(times)
+
+        alone = best([0]) + best([1])
+        assert best([0, 1]) < 1.2 * alone
+    finally:
+        for q in qs:
+            q.close()
+        ctx.close()
