@@ -38,7 +38,9 @@
 // kernel goes on from there.  Everything a barrier waits for is decided from
 // counts and masks that all CTAs hold alike between two barriers, also while one
 // of them is an iteration ahead (cluster_rows.cuh), so all of them leave in the
-// same iteration.
+// same iteration.  The cluster barrier is the kernel's only wait, and unlike the
+// polled ones of the other kernels it has no limit: it ends because every warp
+// of every CTA passes the same barriers in the same order, whatever the data.
 #include "cluster_rows.cuh"
 #include "launch.h"
 

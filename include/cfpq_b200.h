@@ -88,16 +88,25 @@ typedef struct cfpq_closure_opts {
     int32_t max_iterations;  /* 0 = until the fixpoint */
     int32_t use_graph;       /* ENGINE driver, how the iterations are sequenced:
                                 0 (CFPQ_LOOP_HOST)   kernels launched from a host loop
-                                1 (CFPQ_LOOP_DEVICE) no host round trip: one persistent
-                                   cooperative kernel for the whole fixpoint when every
-                                   product is word-level, else the CUDA-graph loop
+                                1 (CFPQ_LOOP_DEVICE) one persistent cooperative kernel for
+                                   the whole fixpoint when every product is word-level,
+                                   else the CUDA-graph loop.  A single AUTO query below
+                                   the selector's size (min_tiles) starts there, or with
+                                   n <= 1024 in one thread-block cluster, and goes on in
+                                   the next loop when its iterations become heavy (one
+                                   host round trip each)
                                 2 (CFPQ_LOOP_GRAPH)  one CUDA graph with a device-side
                                    while condition, one node per kernel */
-    int32_t log_products;    /* CFPQ_LOG_* flags (cfpq_last_kernel_profile, cfpq_product_log) */
+    int32_t log_products;    /* CFPQ_LOG_* flags (cfpq_last_kernel_profile, cfpq_product_log);
+                                with any of them a query does not start in the cluster and
+                                does not change loops on its way */
     int32_t wait_limit;      /* persistent kernel: polls of each bounded device wait (work-item
                                 wait, grid barrier) before it gives up and the closure returns
-                                CFPQ_ERR_TIMEOUT; 0 = default (about one second) */
-    int32_t test_flags;      /* CFPQ_TEST_* hooks for testing the failure paths; 0 in normal use */
+                                CFPQ_ERR_TIMEOUT; 0 = default (about one second).  With a limit a
+                                query does not start in the cluster, whose only wait is the
+                                hardware's cluster barrier: it polls nothing and has no limit */
+    int32_t test_flags;      /* CFPQ_TEST_* hooks for testing the failure paths (not in the
+                                cluster either); 0 in normal use */
     int32_t reserved[1];
 } cfpq_closure_opts;
 
