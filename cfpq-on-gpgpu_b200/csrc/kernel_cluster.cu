@@ -390,20 +390,14 @@ __global__ void __launch_bounds__(kThreads, 1) k_closure_cluster(const __grid_co
             put(a.slots[head].dlt[(t + 1) & 1], dlt + ((par ^ 1) * (size_t)nm + head) * mat, r, w, fresh);
         }
     }
-    for (int o = 16; o > 0; o >>= 1) {
-        reads += __shfl_xor_sync(kFull, reads, o);
-        outw += __shfl_xor_sync(kFull, outw, o);
-        neww += __shfl_xor_sync(kFull, neww, o);
-    }
+    for (int o = 16; o > 0; o >>= 1) reads += __shfl_xor_sync(kFull, reads, o);
+    outw = __reduce_add_sync(kFull, outw);
+    neww = __reduce_add_sync(kFull, neww);
     // per CTA first, in the row collectors (all zero now): an atomic of every warp
     // on the state's words took 6 us
     unsigned long long *const sum = reinterpret_cast<unsigned long long *>(newrow);
-    if (lane == 0 && items) {
-        atomicAdd(sum, (unsigned long long)items);
-        atomicAdd(sum + 1, reads);
-        atomicAdd(sum + 2, (unsigned long long)outw);
-        atomicAdd(sum + 3, (unsigned long long)neww);
-    }
+    const unsigned long long mine_sum = lane == 0 ? items : lane == 1 ? reads : lane == 2 ? outw : neww;
+    if (lane < 4 && mine_sum) atomicAdd(sum + lane, mine_sum);
     __syncthreads();
     if (tid < 5 && sum[tid ? tid - 1 : 0]) {
         unsigned long long *const to = tid == 0   ? &a.st->items_by_variant[2]
