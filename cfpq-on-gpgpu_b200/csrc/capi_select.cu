@@ -14,7 +14,7 @@ void selector_defaults(SelectorParams *sp) {
     memset(sp, 0, sizeof(*sp));
     sp->mode = CFPQ_SELECT_HEURISTIC;
     sp->allowed = (1u << CFPQ_VARIANT_LOP3) | (1u << CFPQ_VARIANT_M4R) | (1u << CFPQ_VARIANT_TC);
-    // Until cfpq_autotune runs: tensor cores for n >= 768 when a tenth of the P
+    // Until cfpq_autotune runs: tensor cores for n >= 705 when a tenth of the P
     // tiles are occupied and 10% of them count (tc_tile_pop).  Measured on
     // whole closures, whose tensor-core terms share one plan and one product
     // launch per iteration: sizes from 16, 12 and 8 tiles on give 13.2, 12.4 and

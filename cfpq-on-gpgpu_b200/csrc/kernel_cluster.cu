@@ -33,7 +33,7 @@
 // The rows that got new bits are collected per CTA and announced once per head.
 //
 // The cost of an iteration grows with the bits of the deltas (row by row, no
-// tiles): when the next iteration would read more than leave_reads rows per
+// tiles; a term that finds nothing in a row group costs about 0.1 us): when the next iteration would read more than leave_reads rows per
 // CTA, the cluster writes matrices and deltas back and leaves; the persistent
 // kernel goes on from there.  Everything a barrier waits for is decided from
 // counts and masks that all CTAs hold alike between two barriers, also while one
