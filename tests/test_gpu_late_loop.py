@@ -1,8 +1,6 @@
 """Heavy small queries go on in the multi-kernel loop: from the host at first, as a
 graph when the same one keeps coming.  Every way gives the oracle's answer, and
 queries of different shapes that take turns do not pay for a graph in each call."""
-import time
-
 import pytest
 
 pytestmark = pytest.mark.gpu
@@ -50,23 +48,21 @@ def test_host_loop_and_graph_give_the_same_answers(pkg, oracle, tmp_path):
 
 
 def test_turns_cost_no_graph(pkg):
-    """A graph takes 310 us to build, each of these queries 500 to 900; by turns they may take 20% more than by
-    themselves (40% with a graph in every call)."""
+    """A graph takes 310 us to build, between the closure's events (the stream waits for it); the loop launched from
+    the host about 100 us more than a graph that is there.  The line lies in the middle."""
     ctx = pkg.capi.Context(0)
     wls = [_dense(pkg, n) for n in (1030, 1100)]
     qs = [pkg.query.PreparedQuery(ctx, wl.grammar, wl.graph) for wl in wls]
     try:
-        def best(order, reps=20):
-            times = []
+        def best(order, reps=40):
+            ms = {i: [] for i in order}
             for _ in range(reps):
-                t0 = time.perf_counter()
                 for i in order:
-                    _call(ctx, qs[i], wls[i])
-                times.append(time.perf_counter() - t0)
-            return min(times)
+                    ms[i].append(_call(ctx, qs[i], wls[i])[0]["device_ms"])
+            return sum(min(v) for v in ms.values())
 
         alone = best([0]) + best([1])
-        assert best([0, 1]) < 1.2 * alone
+        assert best([0, 1]) < alone + 2 * 0.205
     finally:
         for q in qs:
             q.close()
